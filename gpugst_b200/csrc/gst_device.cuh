@@ -39,7 +39,7 @@ constexpr uint32_t FAR_SH = 16;  // far-list byte of the flags word
 __device__ __forceinline__ uint32_t near_sh(uint32_t par) { return par * 8u; }  // near-list byte of a parity
 constexpr int DMAX = 7;
 
-// Job state machine (advanced on the device by k_control once per round).
+// Job state machine (advanced on the device by the control step once per round).
 enum JobState : int32_t { J_FREE = 0, J_INIT, J_SSSP, J_TOUR, J_LB, J_DPSEED, J_DP, J_EXTRACT, J_DONE };
 enum Action : int32_t { A_NONE = 0, A_SSEED, A_WORK, A_SPLIT, A_TOUR, A_LB, A_DSEED, A_EXTRACT };
 
@@ -49,7 +49,7 @@ enum Action : int32_t { A_NONE = 0, A_SSEED, A_WORK, A_SPLIT, A_TOUR, A_LB, A_DS
 enum TaskType : int32_t { T_SPLIT = 0, T_SSEED, T_DSEED, T_TOUR, T_EXTRACT, T_SSSP, T_DP, T_HOP, T_LB, T_SNAP, NT };
 constexpr int MAX_SLOTS = 1024;
 
-// Round-wide work description written by k_control.
+// Round-wide work description written by the control step.
 struct RoundDesc {
   uint32_t items[NT];     // items per task type
   uint32_t task_off[NT + 1];  // warp-task offsets (light types, then heavy types restart at 0)
@@ -64,24 +64,26 @@ struct RoundDesc {
   uint32_t hub_min_deg;   // only items with at least this many arcs under their limit are chunked
   uint32_t hub_min_rest;  // ... and only when at least this many arcs remain under the limit
   uint32_t hub_max_items; // chunk only in rounds with fewer distance items (latency-bound rounds)
-  uint32_t hub_on;        // set by k_control for the current round
+  uint32_t hub_on;        // set by the control step for the current round
   // larger rounds: items of at least hub_big_deg arcs are still chunked in
   // rounds with fewer than hub_max_items2 distance items (0: never)
   uint32_t hub_max_items2, hub_big_deg;
   // ... and only when they exceed 1/hub_share_div of a warp's share of the
   // round's arcs (items x avg_deg / light_warps; 0: no such test)
   uint32_t hub_share_div, avg_deg;
-  uint32_t hub_deg;       // this round's chunking threshold for distance items (INF32: none; k_control)
-  uint32_t grow_chunks;   // DP grows hand hub arcs out this round (set by k_control)
-  uint32_t sssp_w;        // distance items per warp task this round (set by k_control)
-  uint32_t dp_w;          // DP states per warp task this round (set by k_control)
+  uint32_t hub_deg;       // this round's chunking threshold for distance items (INF32: none; control step)
+  uint32_t grow_chunks;   // DP grows hand hub arcs out this round (set by the control step)
+  uint32_t sssp_w;        // distance items per warp task this round (set by the control step)
+  uint32_t dp_w;          // DP states per warp task this round (set by the control step)
   uint32_t dp_wmax;       // largest DP task width (set by the host)
   uint32_t sssp_wmax;     // largest distance task width, at most SSSP_WMAX (set by the host)
   uint32_t merge_stage;   // a DP state with at least this many merge partners stages its row (0: never; host)
   uint32_t light_warps;   // warps of one k_light launch (set by the host)
-  uint32_t nslots;        // 1 + the highest slot in use this round (set by k_control)
+  uint32_t nslots;        // 1 + the highest slot in use this round (set by the control step)
+  uint32_t slot_hi;       // slots at or above it are free (set by the host before each block; 0: unknown)
+  uint32_t small;         // this round is small enough for one cluster (set by the control step)
   // work stealing: a warp that finished its first task takes the next one
-  // from these counters (zeroed by k_control every round)
+  // from these counters (zeroed by the control step every round)
   uint32_t next_light, next_heavy;
 };
 // State of one persistent round launch (k_rounds), written by the host
@@ -99,6 +101,7 @@ struct PersistCtl {
   uint32_t pad;
   unsigned long long timeout_ns;  // limit of every wait
 };
+static_assert(sizeof(RoundDesc) <= 256, "the allocation-free scratch keeps one 256-byte block for it");
 #ifndef GSTB_HUB_CHUNK
 #define GSTB_HUB_CHUNK 256
 #endif
@@ -149,7 +152,7 @@ struct alignas(64) QCtl {
   // sector 5: completion
   uint32_t n_edges;  // extraction: number of tree edges
   uint32_t status;   // extraction: 0 ok, 1 no solution, 2 cycle / inconsistency
-  uint32_t done;     // job finished (set by k_control)
+  uint32_t done;     // job finished (set by the control step)
   uint32_t final_status;  // gst_status of the finished job
   uint32_t cancel;   // set by the host: end the job at the next round (GST_CANCELLED)
   uint32_t early;    // progressive mode: the DP stopped early (1) ...
@@ -196,7 +199,7 @@ struct QDev {
   // place (dist_nx == dist).  Hop-bounded queries run exact (Jacobi)
   // Bellman-Ford rounds over two row buffers: round b reads dist (the exact
   // distances over paths of at most b-1 hops) and writes dist_nx, and
-  // k_control swaps the two after the round.
+  // the control step swaps the two after the round.
   uint32_t* dist_nx;
   // Hop-bounded queries (D >= 2): the round whose exact rows give the
   // incumbent (star_h = floor(D/2): a vertex with every group within star_h
@@ -209,6 +212,8 @@ struct QDev {
   // ratio_num / ratio_den times the proven lower bound (ratio_num 0: exact)
   uint32_t ratio_num, ratio_den;
 };
+
+static_assert(sizeof(QDev) <= 512, "the allocation-free scratch keeps one 512-byte block for it");
 
 struct GraphDev {
   const uint32_t* beg;   // [V+1]

@@ -34,11 +34,11 @@
 #include "gst_device.cuh"
 
 namespace gstb {
-__global__ void k_control(QDev*, QCtl*, int, RoundDesc*, uint32_t*);
 // the round kernels of a block size (128 or 256 threads; null otherwise)
 const void* light_kernel(int threads);
 const void* heavy_kernel(int threads);
 const void* rounds_kernel(int threads);
+const void* small_kernel(int* threads, size_t* smem);
 __global__ void k_init_workspace(uint4*, size_t, uint4*, uint4*, uint32_t, uint4*, size_t);
 }  // namespace gstb
 
@@ -107,6 +107,60 @@ uint32_t env_u32(const char* name, uint32_t def) {
   if (!s || !*s) return def;
   return (uint32_t)strtoul(s, nullptr, 10);
 }
+
+uint32_t avg_degree(const gst_graph* g) {
+  return (uint32_t)std::max<uint64_t>(1, (g->arcs + g->V - 1) / std::max<uint32_t>(1, g->V));
+}
+
+// Launch shape of k_small on the current device: the largest cluster that
+// fits, 16 CTAs (non-portable) or 8.
+struct SmallLaunch {
+  const void* fn = nullptr;
+  int threads = 0, ctas = 0;
+  size_t smem = 0;
+
+  cudaError_t init() {
+    fn = small_kernel(&threads, &smem);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    ctas = 8;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t cfg = config(16, nullptr, &at);
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) ctas = 16;
+    }
+    cudaGetLastError();  // a device without 16-CTA clusters
+    return cudaSuccess;
+  }
+
+  cudaLaunchConfig_t config(int n, cudaStream_t s, cudaLaunchAttribute* at) const {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)n;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)n);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+
+  // One control step, and up to `rounds` small rounds.
+  cudaError_t launch(cudaStream_t s, QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uint32_t* pre, GraphDev g,
+                     uint32_t rounds) const {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = config(ctas, s, &at);
+    void* args[] = {&qd, &ctl, &nslots, &rd, &pre, &g, &rounds};
+    return cudaLaunchKernelExC(&cfg, fn, args);
+  }
+};
+
+// Small rounds that one k_small launch may run: bounds how long a request
+// that arrives meanwhile waits for its admission.
+constexpr uint32_t SMALL_ROUNDS = 64;
 
 struct Job {
   // request
@@ -399,7 +453,7 @@ Layout layout_for(const gst_graph* g, int k, int D, size_t n_members, uint32_t m
 
 // ---------------------------------------------------------------------------
 // Round driver.  Queries occupy slots of device-resident descriptors; every
-// round is k_control -> k_light -> k_heavy, all reading their work from device
+// round is k_small -> k_light -> k_heavy, all reading their work from device
 // memory, so the host launches several rounds back to back and synchronises
 // only to admit new queries and retire finished ones.
 // ---------------------------------------------------------------------------
@@ -429,6 +483,7 @@ class Runner {
     CK(cudaMalloc(&d_qd_, MAX_SLOTS * sizeof(QDev)));
     CK(cudaMalloc(&d_ctl_, MAX_SLOTS * sizeof(QCtl)));
     CK(cudaMalloc(&d_rd_, sizeof(RoundDesc)));
+    CK(small_.init());
     {
       gst_status gs = setup_grids();
       if (gs != GST_OK) return gs;
@@ -447,7 +502,7 @@ class Runner {
       rd.hub_max_items2 = env_u32("GSTB_HUB_MAX_ITEMS2", 8000000);
       rd.hub_big_deg = std::max(32u, env_u32("GSTB_HUB_BIG_DEG", 1024));
       rd.hub_share_div = env_u32("GSTB_HUB_SHARE_DIV", 16);
-      rd.avg_deg = (uint32_t)std::max<uint64_t>(1, (g_->arcs + g_->V - 1) / std::max<uint32_t>(1, g_->V));
+      rd.avg_deg = avg_degree(g_);
       // task widths are sized for the warps resident at once
       rd.light_warps = light_warps();
       rd.sssp_w = 4;
@@ -463,6 +518,7 @@ class Runner {
     CK(cudaMallocHost(&h_rd_, sizeof(RoundDesc)));
     CK(cudaMallocHost(&h_qd_, sizeof(QDev)));
     CK(cudaMallocHost(&h_one_, sizeof(uint32_t)));
+    CK(cudaMallocHost(&h_hi_, 2 * sizeof(uint32_t)));
     CK(cudaMalloc(&d_pc_, sizeof(PersistCtl)));
     CK(cudaMallocHost(&h_pc_, 4 * sizeof(PersistCtl)));  // launch templates, then read-backs, per block half
     memset(h_pc_, 0, 4 * sizeof(PersistCtl));
@@ -543,6 +599,8 @@ class Runner {
     if (h_rd_) cudaFreeHost(h_rd_);
     if (h_qd_) cudaFreeHost(h_qd_);
     if (h_one_) cudaFreeHost(h_one_);
+    if (h_hi_) cudaFreeHost(h_hi_);
+    h_hi_ = nullptr;
     if (h_pc_) cudaFreeHost(h_pc_);
     h_pc_ = nullptr;
     if (d_pc_) cudaFree(d_pc_);
@@ -742,7 +800,7 @@ class Runner {
   }
 
   // Withdraw the admitted job with this tag: its control block's cancel flag
-  // is set stream-ordered after the block in flight, and k_control ends the
+  // is set stream-ordered after the block in flight, and the control step ends the
   // job at its next round with GST_CANCELLED.  False if no admitted job has
   // the tag (the caller checks its pending queue).
   bool cancel_tag(uint64_t tag) {
@@ -870,7 +928,7 @@ class Runner {
 
  private:
   // A block of rounds_per_sync_ rounds as one CUDA graph.  Its arguments are
-  // static: k_control scans every slot and publishes the bound the round
+  // static: the control step publishes the bound the round
   // kernels search, so the graph serves any set of admitted queries.
   gst_status build_round_graph() {
     GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut};
@@ -878,7 +936,7 @@ class Runner {
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     cudaError_t le = cudaSuccess;
     for (uint32_t r = 0; r < rounds_per_sync_; r++) {
-      k_control<<<1, 1024, 0, stream_>>>(d_qd_, d_ctl_, (int)max_slots_, d_rd_, d_pre_);
+      le = small_.launch(stream_, d_qd_, d_ctl_, (int)max_slots_, d_rd_, d_pre_, gd, SMALL_ROUNDS);
       if (le == cudaSuccess) le = launch_light(gd, MAX_SLOTS);
       if (le == cudaSuccess) le = launch_heavy(gd, MAX_SLOTS);
     }
@@ -896,6 +954,10 @@ class Runner {
     const int h = (int)(next_block_ & 1);
     const bool prof = g_->profile;
     blk_persist_[h] = persist_ && !(prof && h_rdtrace_);  // the per-round trace needs separate launches
+    if (nslots_hi_ != slot_hi_) {  // the control steps scan the slots in use
+      slot_hi_ = h_hi_[h] = nslots_hi_;
+      CK(cudaMemcpyAsync(&d_rd_->slot_hi, h_hi_ + h, sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+    }
     if (blk_persist_[h]) {
       // the block's rounds as one persistent launch; its state is reset from
       // this half's pinned template (rewritten only after the block of two
@@ -934,7 +996,8 @@ class Runner {
       const int ns = (int)nslots_hi_;
       cudaEvent_t* pe = ev_prof_[h];
       for (uint32_t r = 0; r < R; r++) {
-        k_control<<<1, 1024, 0, stream_>>>(d_qd_, d_ctl_, ns, d_rd_, d_pre_);
+        // (control steps only: every round runs in the two timed kernels)
+        CK(small_.launch(stream_, d_qd_, d_ctl_, ns, d_rd_, d_pre_, gd, prof ? 0u : SMALL_ROUNDS));
         if (prof) CK(cudaEventRecord(pe[3 * r], stream_));
         CK(launch_light(gd, ns));
         if (prof) CK(cudaEventRecord(pe[3 * r + 1], stream_));
@@ -1025,7 +1088,7 @@ class Runner {
           }
         }
       }
-      // free the slot: a zeroed descriptor is J_FREE for k_control (pinned
+      // free the slot: a zeroed descriptor is J_FREE for the control step (pinned
       // source, so the copy stays asynchronous)
       CK(cudaMemcpyAsync(d_qd_ + s, h_qd_, sizeof(QDev), cudaMemcpyHostToDevice, stream_));
       free_job(j);
@@ -1083,6 +1146,9 @@ class Runner {
   RoundDesc* h_rd_ = nullptr;
   QDev* h_qd_ = nullptr;
   uint32_t* h_one_ = nullptr;  // pinned 1, the source of cancel flags
+  uint32_t* h_hi_ = nullptr;   // pinned [2]: the slot bound sent with a block, per block half
+  uint32_t slot_hi_ = 0;       // the slot bound on the device
+  SmallLaunch small_;
   char* h_stage_ = nullptr;
   char* h_edge_stage_ = nullptr;
   size_t stage_cap_ = 0, stage_off_[2] = {0, 0}, edge_stage_cap_ = 0;
@@ -1978,6 +2044,8 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
   CK(cudaMemsetAsync(q.dflag, 0, L.qbuf - L.dflag, 0));
   // grids: every SM filled to the occupancy limit of each kernel
   int bl = 0, bh = 0;
+  SmallLaunch small;
+  CK(small.init());
   const void* kl = light_kernel(256);
   const void* kh = heavy_kernel(256);
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bl, kl, 256, 0));
@@ -1992,6 +2060,7 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
     rd0.dp_wmax = g->tune.dp_wmax;
     rd0.sssp_wmax = g->tune.sssp_wmax;
     rd0.merge_stage = g->tune.merge_stage;
+    rd0.avg_deg = avg_degree(g);
     CK(cudaMemcpy(d_rd, &rd0, sizeof(RoundDesc), cudaMemcpyHostToDevice));
   }
   // member items v*8 + j, staged through a fixed host array (calls are
@@ -2020,7 +2089,7 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
   uint64_t rounds = 0;
   for (;;) {
     for (uint32_t r = 0; r < R; r++) {
-      k_control<<<1, 1024, 0, 0>>>(d_qd, d_ctl, 1, d_rd, d_pre);
+      CK(small.launch(0, d_qd, d_ctl, 1, d_rd, d_pre, gd, SMALL_ROUNDS));
       {
         int one = 1;
         void* args[] = {&d_qd, &d_rd, &d_pre, &one, &gd};

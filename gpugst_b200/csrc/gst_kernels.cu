@@ -2,9 +2,11 @@
 //
 // Hot path of one query (the reference's DPBF_GPU, code/GPUGST/src/DPQ.cu:275-624,
 // and DPBF_gpu, code/D-GPUGST/src/DPQ.cu:149-269, re-designed).  Every round is
-//   k_control  one thread per query slot: advances the query's state machine
-//              (distance rounds -> tour tables -> DP seed -> DP rounds ->
-//              extraction) and writes the round's work description;
+//   k_small    one cluster: the control step (one thread per query slot
+//              advances the query's state machine: distance rounds -> tour
+//              tables -> DP seed -> DP rounds -> extraction, and the round's
+//              work description is written), then, while rounds are small,
+//              the rounds themselves;
 //   k_light    warp tasks: near-far splits, seeds, tour tables, extraction,
 //              distance items (a vertex with its pending groups; the arcs of
 //              a task's items are relaxed as one flat list by the whole warp:
@@ -661,7 +663,7 @@ __device__ void hop_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_
 
 // A DP task: W items (one per lane) of the round's DP or hop-bounded list.
 // Each lane runs its item's gates; then the warp expands the surviving
-// states one after another.  W is chosen per round by k_control (1 when the
+// states one after another.  W is chosen per round by the control step (1 when the
 // round has few items, so that each state gets a warp of its own; up to 32
 // when it has many, most of which the gates drop).
 __device__ void dp_task(const QDev* qd, const uint32_t* __restrict__ pre, int nslots, uint32_t total,
@@ -712,7 +714,7 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* counter, uint32_t nwarps
 
 // ---------------------------------------------------------------------------
 // Distance items.  A warp task holds W items (a vertex with the mask of its
-// pending groups); W is chosen per round by k_control: 4 when the round has
+// pending groups); W is chosen per round by the control step: 4 when the round has
 // few items (short rounds, low latency), up to 32 when it has many (fewer
 // per-task overheads).  Lanes 0..W-1 read the items' headers in parallel;
 // then the arcs of all items of one query in the task are relaxed as one flat
@@ -1655,6 +1657,9 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c) {
   }
 }
 
+// Bounds of a small round, per warp of the cluster (k_small).
+constexpr uint32_t SMALL_ARCS = 256, SMALL_DP = 2, SMALL_TASKS = 2, SMALL_CHUNKS = 4;
+
 // Shared memory of one control step.
 struct CtlSmem {
   uint32_t wsum[32][NT];  // per-warp inclusive totals, then their scan
@@ -1666,7 +1671,12 @@ struct CtlSmem {
 // (blockDim.x a multiple of 32, at most 1024).  Slots go in chunks of
 // blockDim.x; the per-type prefixes carry from one chunk to the next, so any
 // block size gives the same prefixes.
-__device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uint32_t* pre, CtlSmem& sm) {
+//
+// small_warps: warps of the cluster that runs small rounds itself (0: none).
+// A round that is small for them is laid out for them and marked rd->small.
+__device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uint32_t* pre, CtlSmem& sm,
+                             uint32_t small_warps = 0) {
+  if (rd->slot_hi != 0u) nslots = min(nslots, (int)rd->slot_hi);
   const int tid = threadIdx.x, B = blockDim.x;
   const uint32_t lane = tid & 31, wid = tid >> 5, nw = (uint32_t)B >> 5;
   if (tid == 0) sm.live_cnt = sm.used_hi = 0;
@@ -1738,18 +1748,26 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     __syncthreads();
   }
   if (tid == 0) {
+    const unsigned long long n_sssp = sm.carry[T_SSSP];
+    const unsigned long long n_dp = (unsigned long long)sm.carry[T_DP] + sm.carry[T_HOP];
+    // A small round: at most SMALL_ARCS arcs a warp of the cluster at the
+    // graph's average degree, SMALL_DP states and SMALL_TASKS other tasks
+    const uint32_t n_other = (sm.carry[T_SPLIT] + sm.carry[T_SSEED] + sm.carry[T_DSEED] + 31u) / 32u +
+                             (sm.carry[T_LB] + 31u) / 32u + (sm.carry[T_SNAP] + 31u) / 32u;
+    const bool small = small_warps != 0u && sm.live_cnt != 0u && n_sssp * rd->avg_deg <= SMALL_ARCS * small_warps &&
+                       n_dp <= SMALL_DP * small_warps && n_other <= SMALL_TASKS * small_warps;
+    rd->small = small ? 1u : 0u;
+    const uint32_t lw = small ? small_warps : rd->light_warps;
     // distance items per warp task: 4 while that leaves at most two tasks per
     // light warp, more (up to sssp_wmax) in rounds with many items
     uint32_t w = 4;
-    const unsigned long long n_sssp = sm.carry[T_SSSP];
-    while (w < min(rd->sssp_wmax, SSSP_WMAX) && n_sssp > 2ull * w * rd->light_warps) w <<= 1;
+    while (w < min(rd->sssp_wmax, SSSP_WMAX) && n_sssp > 2ull * w * lw) w <<= 1;
     rd->sssp_w = w;
     // DP states per warp task: 1 while that leaves at most two tasks per
     // light warp (every state gets a warp), more (up to dp_wmax) in rounds
     // with many states
     uint32_t wd = 1;
-    const unsigned long long n_dp = (unsigned long long)sm.carry[T_DP] + sm.carry[T_HOP];
-    while (wd < rd->dp_wmax && n_dp > 2ull * wd * rd->light_warps) wd <<= 1;
+    while (wd < rd->dp_wmax && n_dp > 2ull * wd * lw) wd <<= 1;
     rd->dp_w = wd;
     const uint32_t per_task[NT] = {32, 32, 32, 1, 1, w, wd, wd, 32, 32};
     uint32_t off = 0;
@@ -1790,12 +1808,6 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     // after another on one warp
     rd->grow_chunks = (rd->big != nullptr && (rd->hub_on || wd > 1u)) ? 1u : 0u;
   }
-}
-
-__global__ void __launch_bounds__(1024) k_control(QDev* __restrict__ qd, QCtl* __restrict__ ctl, int nslots,
-                                                  RoundDesc* __restrict__ rd, uint32_t* __restrict__ pre) {
-  __shared__ CtlSmem sm;
-  control_step(qd, ctl, nslots, rd, pre, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -1913,6 +1925,7 @@ __global__ void __launch_bounds__(NW * 32, GSTB_LIGHT_MIN_BLOCKS * 8 / NW)
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t ntasks = __ldcg(&rd->light_tasks);
+  if (ntasks == 0u) return;
   nslots = min(nslots, (int)__ldcg(&rd->nslots));
   // prefixes over slots of the item types with many items, staged once per block
   __shared__ uint32_t s_pre[MAX_SLOTS + 1], s_dp[MAX_SLOTS + 1], s_hop[MAX_SLOTS + 1];
@@ -1952,6 +1965,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t nbig = rd->big ? min(__ldcg(&rd->n_big), rd->big_cap) : 0u;
   const uint32_t ntasks = __ldcg(&rd->heavy_tasks) + nbig;
+  if (ntasks == 0u) return;
   nslots = min(nslots, (int)__ldcg(&rd->nslots));
   __shared__ uint32_t s_lb[MAX_SLOTS + 1];
   __shared__ RelaxHdr s_hub[NW];
@@ -2051,6 +2065,85 @@ struct RoundSmem {
   uint32_t ok, last;
 };
 
+// ---------------------------------------------------------------------------
+// Control and small rounds: one cluster (SMALL_NW warps per CTA), the first
+// kernel of every round.  CTA 0 runs the control step.  While the round it
+// lays out is small the cluster runs it itself and goes on to the next, with
+// hardware cluster barriers between the steps; the first round that is not
+// (or whose arc chunks are too many) is left to the k_light and k_heavy
+// launches that follow.  Most rounds of a query hold a few hundred items and
+// are a chain of dependent accesses: as three launches over the whole GPU
+// such a round costs its launches, a scan of every slot and three grid
+// start-ups.  The cluster also leaves when a query has finished, so that the
+// host sees it, and after `rounds` rounds, so that waiting ones are admitted.
+// Every CTA of a cluster is resident, so the barriers cannot wait for ever.
+// What the rounds write is read with ordinary weak loads after a barrier
+// (release / acquire), as in the persistent launch.  Measured against a
+// one-block control kernel before k_light and k_heavy in every round: one
+// k = 3 query on 10k vertices 1063 -> 746 us, four hop-bounded ones 5360 ->
+// 3837 us, six on 170k vertices 7559 -> 6757 us, a 90-query batch there
+// unchanged (21.8 -> 21.7 ms: its rounds are large).
+// ---------------------------------------------------------------------------
+constexpr int SMALL_NW = 16;
+
+__device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(SMALL_NW * 32, 1)
+    k_small(QDev* qd, QCtl* ctl, int nslots_ctl, RoundDesc* rd, uint32_t* pre, GraphDev g, uint32_t rounds) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  RoundSmem<SMALL_NW>& sm = *reinterpret_cast<RoundSmem<SMALL_NW>*>(s_raw);
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+  // consecutive tasks go to different SMs
+  const uint32_t nwarps = gridDim.x * SMALL_NW, warp = wib * gridDim.x + blockIdx.x;
+  WarpStat& ws = sm.ws[wib];
+  WarpBuf& wb = sm.wb[wib];
+  uint32_t live0 = 0;
+  for (uint32_t r = 0;; r++) {
+    if (blockIdx.x == 0) control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl, r < rounds ? nwarps : 0u);
+    cluster_barrier();
+    const uint32_t live = __ldcg(&rd->n_live);
+    if (r == 0) live0 = live;
+    // every CTA reads the same words, so all of them leave here together
+    if (!__ldcg(&rd->small) || live < live0) return;
+    const int nslots = min(nslots_ctl, (int)__ldcg(&rd->nslots));
+    for (int i = threadIdx.x; i <= nslots; i += blockDim.x) {
+      sm.pre_sssp[i] = __ldcg(pre + T_SSSP * (MAX_SLOTS + 1) + i);
+      sm.pre_dp[i] = __ldcg(pre + T_DP * (MAX_SLOTS + 1) + i);
+      sm.pre_hop[i] = __ldcg(pre + T_HOP * (MAX_SLOTS + 1) + i);
+      sm.pre_lb[i] = __ldcg(pre + T_LB * (MAX_SLOTS + 1) + i);
+    }
+    if (lane == 0) {
+      ws_init(ws);
+      wb_init(wb);
+    }
+    __syncthreads();
+    const uint32_t ntl = __ldcg(&rd->light_tasks), nth = __ldcg(&rd->heavy_tasks);
+    const uint32_t n_lb = __ldcg(&rd->items[T_LB]), n_snap = __ldcg(&rd->items[T_SNAP]);
+    const uint32_t snap0 = __ldcg(&rd->task_off[T_SNAP]);
+    for (uint32_t task = warp; task < ntl + nth; task += nwarps) {
+      if (task < ntl)
+        light_task(qd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
+      else
+        heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].dl);
+    }
+    cluster_barrier();  // the chunk list is complete
+    const uint32_t nbig = rd->big ? min(__ldcg(&rd->n_big), rd->big_cap) : 0u;
+    const bool handover = nbig > SMALL_CHUNKS * nwarps;  // too many for the cluster: k_heavy takes them
+    if (!handover)
+      for (uint32_t i = warp; i < nbig; i += nwarps) chunk_task(qd, rd, g, i, lane, &sm.w[wib].hdr[0], ws, wb);
+    wb_flush(wb, lane);
+    if (lane == 0) ws_flush(ws);
+    cluster_barrier();  // the round's work is done and visible to the next control step
+    if (handover) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) rd->light_tasks = rd->heavy_tasks = 0u;
+      return;
+    }
+  }
+}
+
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, 24 / NW)
     k_rounds(QDev* qd, QCtl* ctl, int nslots_ctl, RoundDesc* rd, uint32_t* pre, GraphDev g, uint32_t R,
@@ -2146,6 +2239,11 @@ const void* light_kernel(int threads) {
 }
 const void* heavy_kernel(int threads) {
   return threads == 128 ? (const void*)k_heavy<4> : threads == 256 ? (const void*)k_heavy<8> : nullptr;
+}
+const void* small_kernel(int* threads, size_t* smem) {
+  *threads = SMALL_NW * 32;
+  *smem = sizeof(RoundSmem<SMALL_NW>);
+  return (const void*)k_small;
 }
 const void* rounds_kernel(int threads) {
   return threads == 128 ? (const void*)k_rounds<4> : threads == 256 ? (const void*)k_rounds<8> : nullptr;
