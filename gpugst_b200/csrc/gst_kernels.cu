@@ -352,17 +352,17 @@ __device__ __forceinline__ void grow_arcs(const QDev& q, const GraphDev& g, uint
 constexpr uint32_t CH_GROW = 1u << 31;  // big-list entry is a DP grow chunk
 constexpr uint32_t CH_HOP = 1u << 30;   // ... of a hop-bounded state
 
-__device__ __forceinline__ bool push_grow_chunks(RoundDesc* rd, uint32_t slot, bool hop, uint32_t s, uint32_t a0,
+__device__ __forceinline__ bool push_grow_chunks(const RoundDesc& sd, RoundDesc* rd, uint32_t slot, bool hop, uint32_t s, uint32_t a0,
                                                  uint32_t a1, uint32_t lane) {
   const uint32_t nch = (a1 - a0 + HUB_CHUNK - 1u) / HUB_CHUNK;
   uint32_t cb = 0;
   if (lane == 0) cb = atomicAdd(&rd->n_big, nch);
   cb = __shfl_sync(0xFFFFFFFFu, cb, 0);
-  const bool fits = cb + nch <= rd->big_cap;
+  const bool fits = cb + nch <= sd.big_cap;
   const uint32_t x = slot | CH_GROW | (hop ? CH_HOP : 0u);
-  for (uint32_t c = lane; c < nch && cb + c < rd->big_cap; c += 32u) {
+  for (uint32_t c = lane; c < nch && cb + c < sd.big_cap; c += 32u) {
     const uint32_t s0 = a0 + c * HUB_CHUNK;
-    rd->big[cb + c] = fits ? make_uint4(x, s, s0, min(s0 + HUB_CHUNK, a1)) : make_uint4(slot, 0u, 0u, 0u);
+    sd.big[cb + c] = fits ? make_uint4(x, s, s0, min(s0 + HUB_CHUNK, a1)) : make_uint4(slot, 0u, 0u, 0u);
   }
   return fits;
 }
@@ -477,7 +477,8 @@ __device__ __forceinline__ bool dp_gate(const QDev& q, uint32_t s, uint32_t& c_o
 }
 
 __device__ void dp_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_t c, uint32_t best, uint32_t lane,
-                          RoundDesc* __restrict__ rd, uint32_t slot, WarpStat& ws, WarpBuf& wb, MergeTile* mt) {
+                          const RoundDesc& sd, RoundDesc* rd, uint32_t slot, WarpStat& ws, WarpBuf& wb,
+                          MergeTile* mt) {
   const int k = q.k;
   const uint32_t K2 = 1u << k, full = (uint32_t)q.full;
   const uint32_t v = s >> k, p = s & (K2 - 1u), comp = full ^ p;
@@ -491,8 +492,8 @@ __device__ void dp_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_t
     const uint32_t lim = best - c;
     const uint32_t a0 = __ldg(g.beg + v);
     uint32_t a1 = arcs_upto(g, v, __ldg(g.beg + v + 1), lim);
-    if (rd->grow_chunks && a1 - a0 >= rd->hub_min_deg &&
-        push_grow_chunks(rd, slot, false, s, a0 + GROW_LOCAL, a1, lane))
+    if (sd.grow_chunks && a1 - a0 >= sd.hub_min_deg &&
+        push_grow_chunks(sd, rd, slot, false, s, a0 + GROW_LOCAL, a1, lane))
       a1 = a0 + GROW_LOCAL;
     grow_arcs(q, g, lane, v, p, comp, c, best, lim, -1, a0, a1, gc, wb);
   }
@@ -508,7 +509,7 @@ __device__ void dp_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_t
   uint32_t merges = 0;
   {
     const uint32_t nsub = (1u << __popc(comp)) - 2u;
-    const bool staged = mt != nullptr && rd->merge_stage != 0u && nsub >= rd->merge_stage;
+    const bool staged = mt != nullptr && sd.merge_stage != 0u && nsub >= sd.merge_stage;
     if (staged) {
       for (uint32_t i = lane; i < K2; i += 32u) {
         mt->cost[i] = (uint32_t)(ld_cg(row + i) >> 32);
@@ -591,7 +592,7 @@ __device__ __forceinline__ bool hop_gate(const QDev& q, uint32_t s, uint32_t& c_
 }
 
 __device__ void hop_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_t c, uint32_t best, uint32_t lane,
-                           RoundDesc* __restrict__ rd, uint32_t slot, WarpStat& ws, WarpBuf& wb) {
+                           const RoundDesc& sd, RoundDesc* rd, uint32_t slot, WarpStat& ws, WarpBuf& wb) {
   const int k = q.k, nd = q.nd, D = q.D;
   const uint32_t K2 = 1u << k, full = (uint32_t)q.full;
   const uint32_t d = s % (uint32_t)nd, vp = s / (uint32_t)nd;
@@ -602,8 +603,8 @@ __device__ void hop_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_
     const uint32_t lim = best - c;
     const uint32_t a0 = __ldg(g.beg + v);
     uint32_t a1 = arcs_upto(g, v, __ldg(g.beg + v + 1), lim);
-    if (rd->grow_chunks && a1 - a0 >= rd->hub_min_deg &&
-        push_grow_chunks(rd, slot, true, s, a0 + GROW_LOCAL, a1, lane))
+    if (sd.grow_chunks && a1 - a0 >= sd.hub_min_deg &&
+        push_grow_chunks(sd, rd, slot, true, s, a0 + GROW_LOCAL, a1, lane))
       a1 = a0 + GROW_LOCAL;
     grow_arcs(q, g, lane, v, p, comp, c, best, lim, (int)d + 1, a0, a1, gc, wb);
   }
@@ -668,7 +669,7 @@ __device__ void hop_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_
 // when it has many, most of which the gates drop).
 __device__ void dp_task(const QDev* qd, const uint32_t* __restrict__ pre, int nslots, uint32_t total,
                         uint32_t task, uint32_t W, bool hop, const GraphDev& g, uint32_t lane,
-                        RoundDesc* __restrict__ rd, WarpStat& ws, WarpBuf& wb, MergeTile* mt) {
+                        const RoundDesc& sd, RoundDesc* rd, WarpStat& ws, WarpBuf& wb, MergeTile* mt) {
   const unsigned FULL = 0xFFFFFFFFu;
   const uint32_t it = task * W + lane;
   const bool valid = lane < W && it < total;
@@ -696,9 +697,9 @@ __device__ void dp_task(const QDev* qd, const uint32_t* __restrict__ pre, int ns
     const uint32_t cc = __shfl_sync(FULL, c, i), bb = __shfl_sync(FULL, best, i);
     const QDev& q = qd[si];
     if (hop)
-      hop_expand(q, g, ss, cc, bb, lane, rd, si, ws, wb);
+      hop_expand(q, g, ss, cc, bb, lane, sd, rd, si, ws, wb);
     else
-      dp_expand(q, g, ss, cc, bb, lane, rd, si, ws, wb, mt);
+      dp_expand(q, g, ss, cc, bb, lane, sd, rd, si, ws, wb, mt);
   }
 }
 
@@ -879,7 +880,7 @@ __device__ __forceinline__ void relax_cnt_add(WarpStat& ws, QCtl* c, RelaxCnt cn
 
 __device__ void sssp_task(const QDev* qd, const uint32_t* __restrict__ pre, int nslots,
                           uint32_t total, uint32_t task, uint32_t W, const GraphDev& g, uint32_t lane, WarpStat& ws,
-                          RoundDesc* __restrict__ rd, RelaxHdr* __restrict__ sh, WarpBuf& wb) {
+                          const RoundDesc& sd, RoundDesc* rd, RelaxHdr* __restrict__ sh, WarpBuf& wb) {
   const unsigned FULL = 0xFFFFFFFFu;
   const uint32_t it = task * W + lane;
   const bool valid = lane < W && it < total;
@@ -948,16 +949,16 @@ __device__ void sssp_task(const QDev* qd, const uint32_t* __restrict__ pre, int 
       n = a1 - b0;
       // hub: hand all but the first HUB_LOCAL arcs to k_heavy in chunks of
       // HUB_CHUNK arcs, one warp each
-      if (n >= rd->hub_deg && n - HUB_LOCAL >= rd->hub_min_rest) {
+      if (n >= sd.hub_deg && n - HUB_LOCAL >= sd.hub_min_rest) {
         const uint32_t st0 = b0 + HUB_LOCAL;
         const uint32_t nch = (a1 - st0 + HUB_CHUNK - 1u) / HUB_CHUNK;
         const uint32_t cb = atomicAdd(&rd->n_big, nch);
-        const bool fits = cb + nch <= rd->big_cap;
+        const bool fits = cb + nch <= sd.big_cap;
         // entries below the cap are always written (empty ranges when the
         // whole run does not fit) so k_heavy never reads a stale entry
-        for (uint32_t c = 0; c < nch && cb + c < rd->big_cap; c++) {
+        for (uint32_t c = 0; c < nch && cb + c < sd.big_cap; c++) {
           const uint32_t s0 = st0 + c * HUB_CHUNK;
-          rd->big[cb + c] = fits ? make_uint4(slot | (rm << 16), v, s0, min(s0 + HUB_CHUNK, a1))
+          sd.big[cb + c] = fits ? make_uint4(slot | (rm << 16), v, s0, min(s0 + HUB_CHUNK, a1))
                                  : make_uint4(slot, v, 0u, 0u);
         }
         if (fits) n = HUB_LOCAL;
@@ -1467,14 +1468,24 @@ __global__ void __launch_bounds__(256) k_init_workspace(uint4* __restrict__ tabl
 // decides this round's action, and publishes per-type item counts as
 // exclusive prefix sums over slots (pre[t][0..nslots]).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void absorb(QDev& q, QCtl& c) {
-  if (c.cancel) {  // the host withdrew the request
+// What a control step reads of a query's control block, loaded at once: read
+// where they are needed, the words would cost a trip to L2 each.
+struct CtlIn {
+  uint32_t best, infeasible, center, n_near, n_far, n_far2, overflow, status, cancel;
+  unsigned long long best_full;
+  __device__ explicit CtlIn(const QCtl& c)
+      : best(c.best), infeasible(c.infeasible), center(c.center), n_near(c.n_near), n_far(c.n_far), n_far2(c.n_far2),
+        overflow(c.overflow), status(c.status), cancel(c.cancel), best_full(c.best_full) {}
+};
+
+__device__ __forceinline__ void absorb(QDev& q, QCtl& c, const CtlIn& in) {
+  if (in.cancel) {  // the host withdrew the request
     q.st = J_DONE;
     c.final_status = 12;  // GST_CANCELLED
     c.done = 1;
     return;
   }
-  if (c.overflow) {
+  if (in.overflow) {
     q.st = J_DONE;
     c.final_status = 6;  // GST_QUEUE_OVERFLOW
     c.done = 1;
@@ -1485,14 +1496,14 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c) {
   switch (q.act) {
     case A_SSEED:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
-      q.n_in = c.n_near;
+      q.n_in = in.n_near;
       q.n_far = 0;
       q.st = J_SSSP;
       break;
     case A_WORK:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
-      q.n_in = c.n_near;
-      q.n_far = c.n_far;
+      q.n_in = in.n_near;
+      q.n_far = in.n_far;
       q.par ^= 1u;  // producers of the round flagged the next items with the other parity
       if (q.st == J_SSSP) {
         q.hops++;
@@ -1511,11 +1522,11 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c) {
     case A_SPLIT:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
       t = q.far_idx; q.far_idx = q.far2_idx; q.far2_idx = t;
-      q.n_in = c.n_near;
-      q.n_far = c.n_far2;
+      q.n_in = in.n_near;
+      q.n_far = in.n_far2;
       break;
     case A_TOUR:
-      q.st = c.infeasible ? J_EXTRACT : J_LB;  // disconnected groups: straight to "no solution"
+      q.st = in.infeasible ? J_EXTRACT : J_LB;  // disconnected groups: straight to "no solution"
       break;
     case A_LB:
       // the bound table is filled in chunks of LB_CHUNK entries per round
@@ -1524,19 +1535,19 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c) {
       break;
     case A_DSEED:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
-      q.n_in = c.n_near;
+      q.n_in = in.n_near;
       q.n_far = 0;
       q.st = J_DP;
       break;
     case A_EXTRACT:
       q.st = J_DONE;
-      c.final_status = c.status == 1 ? 1u : (c.status != 0 ? 8u : 0u);  // NO_SOLUTION / INTERNAL / OK
+      c.final_status = in.status == 1 ? 1u : (in.status != 0 ? 8u : 0u);  // NO_SOLUTION / INTERNAL / OK
       c.done = 1;
       break;
     default:
       break;
   }
-  if (q.act != A_NONE) c.stat[ST_ROUNDS]++;
+  if (q.act != A_NONE) atomicAdd(&c.stat[ST_ROUNDS], 1ull);
   q.act = A_NONE;
 }
 
@@ -1544,12 +1555,12 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c) {
 // <= D has a vertex with all its vertices within ceil(D/2) hops (a centre of
 // the tree), so when the exact rows of that many hops showed no vertex with
 // every group in reach, the query has no solution.
-__device__ __forceinline__ void hop_rounds_done(QDev& q, QCtl& c) {
-  if (q.center_h != 0u && q.center_done && c.center == 0u && c.best == INF32) c.infeasible = 1u;
+__device__ __forceinline__ void hop_rounds_done(QDev& q, QCtl& c, const CtlIn& in) {
+  if (q.center_h != 0u && q.center_done && in.center == 0u && in.best == INF32) c.infeasible = 1u;
   q.dist_nx = q.dist;
 }
 
-__device__ __forceinline__ void decide(QDev& q, QCtl& c) {
+__device__ __forceinline__ void decide(QDev& q, QCtl& c, const CtlIn& in) {
   for (int guard = 0; guard < 8; guard++) {
     switch (q.st) {
       case J_INIT:
@@ -1573,11 +1584,11 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c) {
           // and an unreached vertex cannot join a group
           q.cap1 = BIG;
           q.snap_n = min(q.hops, (uint32_t)q.D - 1u);
-          hop_rounds_done(q, c);
+          hop_rounds_done(q, c, in);
           q.st = J_TOUR;
           continue;
         }
-        if (q.st == J_DP && q.phase == PH_DP && q.ratio_num != 0u && c.best_full != INF64) {
+        if (q.st == J_DP && q.phase == PH_DP && q.ratio_num != 0u && in.best_full != INF64) {
           // Progressive exit (CPUNONHOP.h:730-755, in exact integer
           // arithmetic).  Every state of cost below lo (theta_lo, or theta_hi
           // once the window's near list is empty) has been expanded at its
@@ -1585,7 +1596,7 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c) {
           // the optimum, so an optimum below lo would already be recorded:
           // opt >= min(best_full, lo).  Stop once best_full <= ratio * lo.
           const unsigned long long lo = q.n_in > 0 ? q.theta_lo : q.theta_hi;
-          const unsigned long long bf = c.best_full >> 32;
+          const unsigned long long bf = in.best_full >> 32;
           if (bf * q.ratio_den <= lo * q.ratio_num) {
             c.early = 1u;
             c.lb_exit = (uint32_t)(bf < lo ? bf : lo);
@@ -1601,8 +1612,8 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c) {
         }
         uint32_t next_lo = q.theta_hi;
         // distance rounds only matter up to cap(best); DP rounds up to best
-        unsigned long long limit = c.best;
-        if (q.st == J_SSSP && c.best != INF32) limit = (unsigned long long)c.best * q.cap_num / q.cap_den;
+        unsigned long long limit = in.best;
+        if (q.st == J_SSSP && in.best != INF32) limit = (unsigned long long)in.best * q.cap_num / q.cap_den;
         bool exhausted = q.n_far == 0 || next_lo > limit;
         if (!exhausted) {
           q.theta_lo = next_lo;
@@ -1617,11 +1628,11 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c) {
           // more hops than the snapshots taken are the final distances
           if (q.D >= 0) {
             q.snap_n = min(q.hops, q.D > 0 ? (uint32_t)q.D - 1u : 0u);
-            hop_rounds_done(q, c);
+            hop_rounds_done(q, c, in);
           }
           // every distance below theta_hi is exact and every distance <=
           // cap(best) was discovered; unknown ones are >= min(theta_hi, cap+1)
-          unsigned long long b1 = c.best == INF32 ? (unsigned long long)INF32 : limit + 1;
+          unsigned long long b1 = in.best == INF32 ? (unsigned long long)INF32 : limit + 1;
           unsigned long long cap1 = q.n_far == 0 ? b1 : (q.theta_hi < b1 ? q.theta_hi : b1);
           q.cap1 = (uint32_t)(cap1 < BIG ? cap1 : BIG);
           q.st = J_TOUR;
@@ -1667,49 +1678,69 @@ struct CtlSmem {
   uint32_t live_cnt, used_hi;
 };
 
+// The round's description staged in shared memory (every thread of the block
+// calls it, a barrier follows): a task reads a dozen of its words, one after
+// another, and from L2 each would cost a trip.  `rd` beside a staged copy `sd`
+// is the global one, whose n_big the tasks count up.
+constexpr uint32_t RD_WORDS = sizeof(RoundDesc) / 4;
+static_assert(sizeof(RoundDesc) % 4 == 0, "copied by words");
+__device__ __forceinline__ void stage_rd(RoundDesc& sd, const RoundDesc* rd) {
+  for (uint32_t i = threadIdx.x; i < RD_WORDS; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&sd)[i] = __ldcg(reinterpret_cast<const uint32_t*>(rd) + i);
+}
+
 // One control step over slots [0, nslots) by all threads of one block
 // (blockDim.x a multiple of 32, at most 1024).  Slots go in chunks of
 // blockDim.x; the per-type prefixes carry from one chunk to the next, so any
-// block size gives the same prefixes.
+// block size gives the same prefixes.  Fewer than 32 slots are one warp's
+// work, without the block-wide scan and its barriers.
 //
 // small_warps: warps of the cluster that runs small rounds itself (0: none).
-// A round that is small for them is laid out for them and marked rd->small.
-__device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uint32_t* pre, CtlSmem& sm,
+// A round that is small for them is laid out for them and marked small.
+// sd: the block's staged copy of the round description; on return it holds
+// the new one, which has been written to *rd.
+__device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uint32_t* pre, CtlSmem& sm, RoundDesc& sd,
                              uint32_t small_warps = 0) {
-  if (rd->slot_hi != 0u) nslots = min(nslots, (int)rd->slot_hi);
   const int tid = threadIdx.x, B = blockDim.x;
   const uint32_t lane = tid & 31, wid = tid >> 5, nw = (uint32_t)B >> 5;
+  stage_rd(sd, rd);
   if (tid == 0) sm.live_cnt = sm.used_hi = 0;
   if (tid < NT) sm.carry[tid] = 0;
   __syncthreads();
+  if (sd.slot_hi != 0u) nslots = min(nslots, (int)sd.slot_hi);
+  const bool one_warp = nslots < 32;
   for (int base = 0; base <= nslots; base += B) {
+    if (one_warp && wid != 0u) break;
     const int s = base + tid;
     uint32_t cnt[NT];
 #pragma unroll
     for (int t = 0; t < NT; t++) cnt[t] = 0;
-    // the state alone first: most slots are free when the scan covers them all
-    const int32_t st0 = s < nslots ? qd[s].st : J_FREE;
-    if (st0 != J_FREE) atomicMax(&sm.used_hi, (uint32_t)s + 1u);
-    if (st0 != J_FREE && st0 != J_DONE) {
+    if (s < nslots) {
+      // (a free slot's words are loaded too: its state alone first would put
+      // another trip to L2 in front of every live one's)
       QDev q = qd[s];
       QCtl& c = ctl[s];
-      absorb(q, c);
-      if (q.st != J_DONE) decide(q, c);
-      switch (q.act) {
-        case A_SSEED: cnt[T_SSEED] = q.n_members; break;
-        case A_DSEED: cnt[T_DSEED] = q.n_members; break;
-        case A_SPLIT: cnt[T_SPLIT] = q.n_far; break;
-        case A_TOUR: cnt[T_TOUR] = 1; break;
-        case A_LB: cnt[T_LB] = min(q.nv - q.lb_off, LB_CHUNK); break;
-        case A_EXTRACT: cnt[T_EXTRACT] = 1; break;
-        case A_WORK:
-          cnt[q.phase == PH_SSSP ? T_SSSP : (q.phase == PH_DP ? T_DP : T_HOP)] = q.n_in;
-          break;
-        default: break;
+      const CtlIn in(c);
+      if (q.st != J_FREE) atomicMax(&sm.used_hi, (uint32_t)s + 1u);
+      if (q.st != J_FREE && q.st != J_DONE) {
+        absorb(q, c, in);
+        if (q.st != J_DONE) decide(q, c, in);
+        switch (q.act) {
+          case A_SSEED: cnt[T_SSEED] = q.n_members; break;
+          case A_DSEED: cnt[T_DSEED] = q.n_members; break;
+          case A_SPLIT: cnt[T_SPLIT] = q.n_far; break;
+          case A_TOUR: cnt[T_TOUR] = 1; break;
+          case A_LB: cnt[T_LB] = min(q.nv - q.lb_off, LB_CHUNK); break;
+          case A_EXTRACT: cnt[T_EXTRACT] = 1; break;
+          case A_WORK:
+            cnt[q.phase == PH_SSSP ? T_SSSP : (q.phase == PH_DP ? T_DP : T_HOP)] = q.n_in;
+            break;
+          default: break;
+        }
+        if (q.snap_h) cnt[T_SNAP] = q.nv;  // copy the distance rows of round snap_h
+        if (q.st != J_DONE) atomicAdd(&sm.live_cnt, 1u);
+        qd[s] = q;
       }
-      if (q.snap_h) cnt[T_SNAP] = q.nv;  // copy the distance rows of round snap_h
-      if (q.st != J_DONE) atomicAdd(&sm.live_cnt, 1u);
-      qd[s] = q;
     }
     // exclusive scan over the chunk's slots, per task type
     uint32_t incl[NT];
@@ -1723,6 +1754,14 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
       }
       incl[t] = x;
       if (lane == 31) sm.wsum[wid][t] = x;
+    }
+    if (one_warp) {
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        if (s <= nslots) pre[t * (MAX_SLOTS + 1) + s] = incl[t] - cnt[t];
+        if (lane == 31) sm.carry[t] = incl[t];
+      }
+      break;
     }
     __syncthreads();
     if (wid == 0) {
@@ -1747,6 +1786,7 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     if (tid < NT) sm.carry[tid] += sm.wsum[nw - 1][tid];
     __syncthreads();
   }
+  __syncwarp();
   if (tid == 0) {
     const unsigned long long n_sssp = sm.carry[T_SSSP];
     const unsigned long long n_dp = (unsigned long long)sm.carry[T_DP] + sm.carry[T_HOP];
@@ -1754,60 +1794,64 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     // graph's average degree, SMALL_DP states and SMALL_TASKS other tasks
     const uint32_t n_other = (sm.carry[T_SPLIT] + sm.carry[T_SSEED] + sm.carry[T_DSEED] + 31u) / 32u +
                              (sm.carry[T_LB] + 31u) / 32u + (sm.carry[T_SNAP] + 31u) / 32u;
-    const bool small = small_warps != 0u && sm.live_cnt != 0u && n_sssp * rd->avg_deg <= SMALL_ARCS * small_warps &&
+    const bool small = small_warps != 0u && sm.live_cnt != 0u && n_sssp * sd.avg_deg <= SMALL_ARCS * small_warps &&
                        n_dp <= SMALL_DP * small_warps && n_other <= SMALL_TASKS * small_warps;
-    rd->small = small ? 1u : 0u;
-    const uint32_t lw = small ? small_warps : rd->light_warps;
+    sd.small = small ? 1u : 0u;
+    const uint32_t lw = small ? small_warps : sd.light_warps;
     // distance items per warp task: 4 while that leaves at most two tasks per
     // light warp, more (up to sssp_wmax) in rounds with many items
     uint32_t w = 4;
-    while (w < min(rd->sssp_wmax, SSSP_WMAX) && n_sssp > 2ull * w * lw) w <<= 1;
-    rd->sssp_w = w;
+    while (w < min(sd.sssp_wmax, SSSP_WMAX) && n_sssp > 2ull * w * lw) w <<= 1;
+    sd.sssp_w = w;
     // DP states per warp task: 1 while that leaves at most two tasks per
     // light warp (every state gets a warp), more (up to dp_wmax) in rounds
     // with many states
     uint32_t wd = 1;
-    while (wd < rd->dp_wmax && n_dp > 2ull * wd * lw) wd <<= 1;
-    rd->dp_w = wd;
+    while (wd < sd.dp_wmax && n_dp > 2ull * wd * lw) wd <<= 1;
+    sd.dp_w = wd;
     const uint32_t per_task[NT] = {32, 32, 32, 1, 1, w, wd, wd, 32, 32};
     uint32_t off = 0;
+#pragma unroll
     for (int t = 0; t < NT; t++) {
       uint32_t tot = sm.carry[t];
-      rd->items[t] = tot;
+      sd.items[t] = tot;
       if (t == T_LB) {
-        rd->light_tasks = off;
+        sd.light_tasks = off;
         off = 0;
       }
-      rd->task_off[t] = off;
+      sd.task_off[t] = off;
       off += (tot + per_task[t] - 1) / per_task[t];
     }
-    rd->task_off[NT] = off;
-    rd->heavy_tasks = off;
-    rd->n_live = sm.live_cnt;
-    rd->nslots = sm.used_hi;  // slots the round kernels search (all later ones are free)
-    rd->n_big = 0;
-    rd->next_light = 0;
-    rd->next_heavy = 0;
+    sd.task_off[NT] = off;
+    sd.heavy_tasks = off;
+    sd.n_live = sm.live_cnt;
+    sd.nslots = sm.used_hi;  // slots the round kernels search (all later ones are free)
+    sd.n_big = 0;
+    sd.next_light = 0;
+    sd.next_heavy = 0;
     // hub chunking pays off only when the round is too small to fill the GPU
-    const uint32_t n_items = rd->items[T_SSSP] + rd->items[T_DP] + rd->items[T_HOP];
-    rd->hub_on = (rd->big != nullptr && n_items < rd->hub_max_items) ? 1u : 0u;
+    const uint32_t n_items = (uint32_t)(n_sssp + n_dp);
+    sd.hub_on = (sd.big != nullptr && n_items < sd.hub_max_items) ? 1u : 0u;
     // distance items: every hub in small rounds; in larger ones (a single
     // query's dense rounds) only the biggest hubs, whose one warp would
     // otherwise finish long after the rest: at least hub_big_deg arcs and
     // more than 1/hub_share_div of a warp's share of the round's arcs
-    uint32_t big_deg = rd->hub_big_deg;
-    if (rd->hub_share_div != 0u) {
+    uint32_t big_deg = sd.hub_big_deg;
+    if (sd.hub_share_div != 0u) {
       const unsigned long long share =
-          (unsigned long long)n_items * rd->avg_deg / max(1u, rd->light_warps) / rd->hub_share_div;
+          (unsigned long long)n_items * sd.avg_deg / max(1u, sd.light_warps) / sd.hub_share_div;
       big_deg = (uint32_t)max((unsigned long long)big_deg, min(share, (unsigned long long)INF32 - 1ull));
     }
-    rd->hub_deg = rd->hub_on ? rd->hub_min_deg
-                             : ((rd->big != nullptr && n_items < rd->hub_max_items2) ? big_deg : INF32);
+    sd.hub_deg = sd.hub_on ? sd.hub_min_deg
+                           : ((sd.big != nullptr && n_items < sd.hub_max_items2) ? big_deg : INF32);
     // DP tasks that hold several states hand their hub grows out in every
     // round: a task with a few hub states would otherwise grow them one
     // after another on one warp
-    rd->grow_chunks = (rd->big != nullptr && (rd->hub_on || wd > 1u)) ? 1u : 0u;
+    sd.grow_chunks = (sd.big != nullptr && (sd.hub_on || wd > 1u)) ? 1u : 0u;
   }
+  __syncthreads();
+  for (uint32_t i = tid; i < RD_WORDS; i += B)
+    reinterpret_cast<uint32_t*>(rd)[i] = reinterpret_cast<const uint32_t*>(&sd)[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -1818,20 +1862,19 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
 // Light task `task` (types T_SPLIT .. T_HOP: splits, seeds, tour tables,
 // extraction, distance items, DP states).  s_pre / s_dp / s_hop: the per-slot
 // prefixes of the distance, DP and hop items, staged in shared memory.
-__device__ __forceinline__ void light_task(const QDev* qd, RoundDesc* rd, const uint32_t* pre,
+__device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, RoundDesc* rd, const uint32_t* pre,
                                            const uint32_t* s_pre, const uint32_t* s_dp, const uint32_t* s_hop,
                                            int nslots, const GraphDev& g, uint32_t task, uint32_t lane,
                                            WarpStat& ws, WarpBuf& wb, WarpScratch& sc) {
   int t = 0;
-  while (t < T_HOP && task >= __ldcg(&rd->task_off[t + 1])) t++;
-  const uint32_t local = task - __ldcg(&rd->task_off[t]);
+  while (t < T_HOP && task >= sd.task_off[t + 1]) t++;
+  const uint32_t local = task - sd.task_off[t];
   const uint32_t* P = pre + t * (MAX_SLOTS + 1);
-  const uint32_t total = __ldcg(&rd->items[t]);
+  const uint32_t total = sd.items[t];
   if (t == T_SSSP) {
-    sssp_task(qd, s_pre, nslots, total, local, __ldcg(&rd->sssp_w), g, lane, ws, rd, sc.hdr, wb);
+    sssp_task(qd, s_pre, nslots, total, local, sd.sssp_w, g, lane, ws, sd, rd, sc.hdr, wb);
   } else if (t == T_DP || t == T_HOP) {
-    dp_task(qd, t == T_DP ? s_dp : s_hop, nslots, total, local, __ldcg(&rd->dp_w), t == T_HOP, g, lane, rd, ws, wb,
-            &sc.mg);
+    dp_task(qd, t == T_DP ? s_dp : s_hop, nslots, total, local, sd.dp_w, t == T_HOP, g, lane, sd, rd, ws, wb, &sc.mg);
   } else if (t == T_TOUR) {
     tour_warp(qd[find_slot(P, nslots, local)], lane);
   } else if (t == T_EXTRACT) {
@@ -1903,9 +1946,9 @@ __device__ __forceinline__ void heavy_static_task(const QDev* qd, const uint32_t
 
 // Arc chunk `i` that a light task handed over this round (hub vertex of a
 // distance item, or a high-degree DP state's grow).
-__device__ __forceinline__ void chunk_task(const QDev* qd, const RoundDesc* rd, const GraphDev& g, uint32_t i,
+__device__ __forceinline__ void chunk_task(const QDev* qd, const RoundDesc& sd, const GraphDev& g, uint32_t i,
                                            uint32_t lane, RelaxHdr* hub, WarpStat& ws, WarpBuf& wb) {
-  const uint4 it = __ldcg(rd->big + i);
+  const uint4 it = __ldcg(sd.big + i);
   if (it.x & CH_GROW)
     grow_chunk(qd, it, g, lane, ws, wb);
   else
@@ -1924,9 +1967,12 @@ __global__ void __launch_bounds__(NW * 32, GSTB_LIGHT_MIN_BLOCKS * 8 / NW)
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t ntasks = __ldcg(&rd->light_tasks);
+  __shared__ RoundDesc sd;
+  stage_rd(sd, rd);
+  __syncthreads();
+  const uint32_t ntasks = sd.light_tasks;
   if (ntasks == 0u) return;
-  nslots = min(nslots, (int)__ldcg(&rd->nslots));
+  nslots = min(nslots, (int)sd.nslots);
   // prefixes over slots of the item types with many items, staged once per block
   __shared__ uint32_t s_pre[MAX_SLOTS + 1], s_dp[MAX_SLOTS + 1], s_hop[MAX_SLOTS + 1];
   __shared__ WarpScratch s_sc[NW];
@@ -1949,7 +1995,7 @@ __global__ void __launch_bounds__(NW * 32, GSTB_LIGHT_MIN_BLOCKS * 8 / NW)
 #else
   for (uint32_t task = warp; task < ntasks; task += nwarps)
 #endif
-    light_task(qd, rd, pre, s_pre, s_dp, s_hop, nslots, g, task, lane, ws, wb, s_sc[threadIdx.x >> 5]);
+    light_task(qd, sd, rd, pre, s_pre, s_dp, s_hop, nslots, g, task, lane, ws, wb, s_sc[threadIdx.x >> 5]);
   wb_flush(wb, lane);
   if (lane == 0) ws_flush(ws);
 }
@@ -1963,10 +2009,13 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t nbig = rd->big ? min(__ldcg(&rd->n_big), rd->big_cap) : 0u;
-  const uint32_t ntasks = __ldcg(&rd->heavy_tasks) + nbig;
+  __shared__ RoundDesc sd;
+  stage_rd(sd, rd);
+  __syncthreads();
+  const uint32_t nbig = sd.big ? min(sd.n_big, sd.big_cap) : 0u;
+  const uint32_t ntasks = sd.heavy_tasks + nbig;
   if (ntasks == 0u) return;
-  nslots = min(nslots, (int)__ldcg(&rd->nslots));
+  nslots = min(nslots, (int)sd.nslots);
   __shared__ uint32_t s_lb[MAX_SLOTS + 1];
   __shared__ RelaxHdr s_hub[NW];
   __shared__ uint32_t s_dl[NW][KMAX][32];  // bound rows: each lane's capped distances
@@ -1980,15 +2029,15 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
   }
   for (int i = threadIdx.x; i <= nslots; i += blockDim.x) s_lb[i] = __ldcg(pre + T_LB * (MAX_SLOTS + 1) + i);
   __syncthreads();
-  const uint32_t n_lb = __ldcg(&rd->items[T_LB]), n_snap = __ldcg(&rd->items[T_SNAP]);
-  const uint32_t snap0 = __ldcg(&rd->task_off[T_SNAP]);  // heavy tasks before the snapshot rows
+  const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP];
+  const uint32_t snap0 = sd.task_off[T_SNAP];  // heavy tasks before the snapshot rows
 #if GSTB_STEAL
   for (uint32_t task = warp; task < ntasks; task = next_task(&rd->next_heavy, nwarps, lane)) {
 #else
   for (uint32_t task = warp; task < ntasks; task += nwarps) {
 #endif
     if (task < nbig)
-      chunk_task(qd, rd, g, task, lane, &s_hub[threadIdx.x >> 5], ws, wb);
+      chunk_task(qd, sd, g, task, lane, &s_hub[threadIdx.x >> 5], ws, wb);
     else
       heavy_static_task(qd, pre, s_lb, nslots, task - nbig, snap0, n_lb, n_snap, lane, s_dl[threadIdx.x >> 5]);
   }
@@ -2062,6 +2111,7 @@ struct RoundSmem {
   WarpStat ws[NW];
   WarpBuf wb[NW];
   CtlSmem ctl;
+  RoundDesc rd;
   uint32_t ok, last;
 };
 
@@ -2085,6 +2135,12 @@ struct RoundSmem {
 // unchanged (21.8 -> 21.7 ms: its rounds are large).
 // ---------------------------------------------------------------------------
 constexpr int SMALL_NW = 16;
+constexpr int SMALL_SLOTS = 8;  // query descriptors kept in shared memory
+
+struct SmallSmem {
+  RoundSmem<SMALL_NW> r;
+  QDev qd[SMALL_SLOTS];
+};
 
 __device__ __forceinline__ void cluster_barrier() {
   __syncwarp();
@@ -2094,48 +2150,68 @@ __device__ __forceinline__ void cluster_barrier() {
 __global__ void __launch_bounds__(SMALL_NW * 32, 1)
     k_small(QDev* qd, QCtl* ctl, int nslots_ctl, RoundDesc* rd, uint32_t* pre, GraphDev g, uint32_t rounds) {
   extern __shared__ __align__(16) unsigned char s_raw[];
-  RoundSmem<SMALL_NW>& sm = *reinterpret_cast<RoundSmem<SMALL_NW>*>(s_raw);
+  SmallSmem& ss = *reinterpret_cast<SmallSmem*>(s_raw);
+  RoundSmem<SMALL_NW>& sm = ss.r;
+  const RoundDesc& sd = sm.rd;
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
   // consecutive tasks go to different SMs
   const uint32_t nwarps = gridDim.x * SMALL_NW, warp = wib * gridDim.x + blockIdx.x;
   WarpStat& ws = sm.ws[wib];
   WarpBuf& wb = sm.wb[wib];
   uint32_t live0 = 0;
+  if (lane == 0) {
+    ws_init(ws);
+    wb_init(wb);
+  }
   for (uint32_t r = 0;; r++) {
-    if (blockIdx.x == 0) control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl, r < rounds ? nwarps : 0u);
+    if (blockIdx.x == 0) control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl, sm.rd, r < rounds ? nwarps : 0u);
     cluster_barrier();
-    const uint32_t live = __ldcg(&rd->n_live);
-    if (r == 0) live0 = live;
-    // every CTA reads the same words, so all of them leave here together
-    if (!__ldcg(&rd->small) || live < live0) return;
-    const int nslots = min(nslots_ctl, (int)__ldcg(&rd->nslots));
-    for (int i = threadIdx.x; i <= nslots; i += blockDim.x) {
+    // the round's description, the first slots' prefixes and descriptors in
+    // one trip to L2 (with few slots in use they are all there is)
+    stage_rd(sm.rd, rd);
+    auto stage_pre = [&](int i) {
       sm.pre_sssp[i] = __ldcg(pre + T_SSSP * (MAX_SLOTS + 1) + i);
       sm.pre_dp[i] = __ldcg(pre + T_DP * (MAX_SLOTS + 1) + i);
       sm.pre_hop[i] = __ldcg(pre + T_HOP * (MAX_SLOTS + 1) + i);
       sm.pre_lb[i] = __ldcg(pre + T_LB * (MAX_SLOTS + 1) + i);
-    }
-    if (lane == 0) {
-      ws_init(ws);
-      wb_init(wb);
-    }
+    };
+    if (threadIdx.x <= SMALL_SLOTS) stage_pre(threadIdx.x);
+    const uint32_t qw = min(nslots_ctl, SMALL_SLOTS) * (uint32_t)(sizeof(QDev) / 8);
+    for (uint32_t i = threadIdx.x; i < qw; i += blockDim.x)
+      reinterpret_cast<unsigned long long*>(ss.qd)[i] = __ldcg(reinterpret_cast<const unsigned long long*>(qd) + i);
     __syncthreads();
-    const uint32_t ntl = __ldcg(&rd->light_tasks), nth = __ldcg(&rd->heavy_tasks);
-    const uint32_t n_lb = __ldcg(&rd->items[T_LB]), n_snap = __ldcg(&rd->items[T_SNAP]);
-    const uint32_t snap0 = __ldcg(&rd->task_off[T_SNAP]);
+    if (r == 0) live0 = sd.n_live;
+    // every CTA reads the same words, so all of them leave here together
+    if (!sd.small || sd.n_live < live0) return;
+    const int nslots = min(nslots_ctl, (int)sd.nslots);
+    const QDev* q = qd;
+    if (nslots <= SMALL_SLOTS) {
+      q = ss.qd;
+    } else {
+      for (int i = SMALL_SLOTS + 1 + threadIdx.x; i <= nslots; i += blockDim.x) stage_pre(i);
+      __syncthreads();
+    }
+    const uint32_t ntl = sd.light_tasks, nth = sd.heavy_tasks;
+    const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP], snap0 = sd.task_off[T_SNAP];
     for (uint32_t task = warp; task < ntl + nth; task += nwarps) {
       if (task < ntl)
-        light_task(qd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
+        light_task(q, sd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
       else
-        heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].dl);
+        heavy_static_task(q, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].dl);
     }
-    cluster_barrier();  // the chunk list is complete
-    const uint32_t nbig = rd->big ? min(__ldcg(&rd->n_big), rd->big_cap) : 0u;
-    const bool handover = nbig > SMALL_CHUNKS * nwarps;  // too many for the cluster: k_heavy takes them
-    if (!handover)
-      for (uint32_t i = warp; i < nbig; i += nwarps) chunk_task(qd, rd, g, i, lane, &sm.w[wib].hdr[0], ws, wb);
+    bool handover = false;
+    if (sd.hub_deg != INF32 || sd.grow_chunks != 0u) {
+      cluster_barrier();  // the chunk list is complete
+      const uint32_t nbig = sd.big ? min(__ldcg(&rd->n_big), sd.big_cap) : 0u;
+      handover = nbig > SMALL_CHUNKS * nwarps;  // too many for the cluster: k_heavy takes them
+      if (!handover)
+        for (uint32_t i = warp; i < nbig; i += nwarps) chunk_task(q, sd, g, i, lane, &sm.w[wib].hdr[0], ws, wb);
+    }
     wb_flush(wb, lane);
-    if (lane == 0) ws_flush(ws);
+    if (lane == 0) {
+      wb.q = nullptr;  // the descriptors are staged again
+      ws_flush(ws);
+    }
     cluster_barrier();  // the round's work is done and visible to the next control step
     if (handover) {
       if (blockIdx.x == 0 && threadIdx.x == 0) rd->light_tasks = rd->heavy_tasks = 0u;
@@ -2156,7 +2232,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
   WarpBuf& wb = sm.wb[wib];
   uint32_t p1 = 0;  // rounds with a chunk phase so far (the same in every block)
   if (blockIdx.x == 0) {
-    control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl);
+    control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl, sm.rd);
     __syncthreads();
     if (threadIdx.x == 0) publish(pc, 1u);
   }
@@ -2164,10 +2240,13 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     if (threadIdx.x == 0) sm.ok = wait_geq(&pc->epoch, r + 1u, pc, 1u) ? 1u : 0u;
     __syncthreads();
     if (!sm.ok) return;
+    stage_rd(sm.rd, rd);
+    __syncthreads();
+    const RoundDesc& sd = sm.rd;
     // a round with no live query does nothing, nor do the rest: every block
     // reads the same count, so every block leaves here together
-    if (__ldcg(&rd->n_live) == 0u) return;
-    const int nslots = min(nslots_ctl, (int)__ldcg(&rd->nslots));
+    if (sd.n_live == 0u) return;
+    const int nslots = min(nslots_ctl, (int)sd.nslots);
     for (int i = threadIdx.x; i <= nslots; i += blockDim.x) {
       sm.pre_sssp[i] = __ldcg(pre + T_SSSP * (MAX_SLOTS + 1) + i);
       sm.pre_dp[i] = __ldcg(pre + T_DP * (MAX_SLOTS + 1) + i);
@@ -2179,22 +2258,21 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
       wb_init(wb);
     }
     __syncthreads();
-    const uint32_t ntl = __ldcg(&rd->light_tasks), nth = __ldcg(&rd->heavy_tasks);
-    const uint32_t n_lb = __ldcg(&rd->items[T_LB]), n_snap = __ldcg(&rd->items[T_SNAP]);
-    const uint32_t snap0 = __ldcg(&rd->task_off[T_SNAP]);
+    const uint32_t ntl = sd.light_tasks, nth = sd.heavy_tasks;
+    const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP], snap0 = sd.task_off[T_SNAP];
     // light tasks, then the static heavy ones, as one list dealt out over
     // the warps (two lists dealt out one after the other would leave the
     // warps with the heaviest light tasks also the first heavy ones)
     for (uint32_t task = warp; task < ntl + nth; task += nwarps) {
       if (task < ntl)
-        light_task(qd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
+        light_task(qd, sd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
       else
         heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].dl);
     }
     // phase 1 done in this block: its chunk entries are written.  Rounds
     // that hand out no chunks (every block reads the same flags) skip the
     // grid-wide wait for the others
-    if (rd->big != nullptr && (__ldcg(&rd->hub_deg) != INF32 || __ldcg(&rd->grow_chunks) != 0u)) {
+    if (sd.big != nullptr && (sd.hub_deg != INF32 || sd.grow_chunks != 0u)) {
       p1++;
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -2205,8 +2283,8 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     }
     __syncthreads();
     if (sm.ok) {
-      const uint32_t nbig = rd->big ? min(__ldcg(&rd->n_big), rd->big_cap) : 0u;
-      for (uint32_t i = warp; i < nbig; i += nwarps) chunk_task(qd, rd, g, i, lane, &sm.w[wib].hdr[0], ws, wb);
+      const uint32_t nbig = sd.big ? min(__ldcg(&rd->n_big), sd.big_cap) : 0u;
+      for (uint32_t i = warp; i < nbig; i += nwarps) chunk_task(qd, sd, g, i, lane, &sm.w[wib].hdr[0], ws, wb);
     }
     wb_flush(wb, lane);
     if (lane == 0) ws_flush(ws);
@@ -2223,7 +2301,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     }
     __syncthreads();
     if (sm.last && r + 1u < R) {
-      control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl);
+      control_step(qd, ctl, nslots_ctl, rd, pre, sm.ctl, sm.rd);
       __syncthreads();
       if (threadIdx.x == 0) publish(pc, r + 2u);
     }
@@ -2242,7 +2320,7 @@ const void* heavy_kernel(int threads) {
 }
 const void* small_kernel(int* threads, size_t* smem) {
   *threads = SMALL_NW * 32;
-  *smem = sizeof(RoundSmem<SMALL_NW>);
+  *smem = sizeof(SmallSmem);
   return (const void*)k_small;
 }
 const void* rounds_kernel(int threads) {
