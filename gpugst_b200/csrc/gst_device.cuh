@@ -193,7 +193,7 @@ struct QDev {
   uint32_t hops;     // distance rounds done (hop-bounded queries stop after D)
   uint32_t snap_h;   // distance round whose rows k_heavy copies to snap this round (0: none)
   uint32_t snap_n;   // snapshots taken (rows for b hops: snap[b-1] if b <= snap_n, else dist)
-  uint32_t pad_s;
+  uint32_t win_items;  // items of the current window's rounds so far
   uint32_t* snap;    // [D-1][V][8] (hop-bounded queries)
   // Distance rows written by a distance round.  Unbounded queries relax in
   // place (dist_nx == dist).  Hop-bounded queries run exact (Jacobi)
