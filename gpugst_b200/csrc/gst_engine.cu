@@ -39,7 +39,7 @@ const void* light_kernel(int threads);
 const void* heavy_kernel(int threads);
 const void* rounds_kernel(int threads);
 const void* small_kernel(int* threads, size_t* smem);
-__global__ void k_init_workspace(uint4*, size_t, uint4*, uint4*, uint32_t, uint4*, size_t);
+__global__ void k_init_workspace(uint4*, uint4*, uint32_t, uint4*, size_t);
 }  // namespace gstb
 
 using namespace gstb;
@@ -157,6 +157,15 @@ struct SmallLaunch {
     return cudaLaunchKernelExC(&cfg, fn, args);
   }
 };
+
+// What must hold before a query's first round: distances unknown with no
+// group pending and, where the bound-row pass does not clear them (k < 3), no
+// state flag set (the flags' span is 256-aligned).
+void init_workspace(const gst_graph* g, const QDev& q, size_t dflag_vec, cudaStream_t s) {
+  k_init_workspace<<<(unsigned)g->num_sms * 8u, 256, 0, s>>>(
+      reinterpret_cast<uint4*>(q.dist), q.dist_nx != q.dist ? reinterpret_cast<uint4*>(q.dist_nx) : nullptr, q.nv,
+      reinterpret_cast<uint4*>(q.dflag), q.k < 3 ? dflag_vec : 0);
+}
 
 // Small rounds that one k_small launch may run: bounds how long a request
 // that arrives meanwhile waits for its admission.
@@ -766,13 +775,7 @@ class Runner {
     memset(&j->ctl, 0, sizeof(j->ctl));
     j->ctl.best = INF32;
     j->ctl.best_full = INF64;
-    // state table INF, distances unknown with no group pending, no state
-    // flag set: one launch (the byte counts are multiples of 16: the table
-    // holds an even number of 8-byte words, the flags span is 256-aligned)
-    k_init_workspace<<<(unsigned)g_->num_sms * 8u, 256, 0, stream_>>>(
-        reinterpret_cast<uint4*>(q.table), (size_t)g_->V * j->WT * 8 / 16, reinterpret_cast<uint4*>(q.dist),
-        q.dist_nx != q.dist ? reinterpret_cast<uint4*>(q.dist_nx) : nullptr, g_->V,
-        reinterpret_cast<uint4*>(q.dflag), (L.qbuf - L.dflag) / 16);
+    init_workspace(g_, q, (L.qbuf - L.dflag) / 16, stream_);
     g_->launches++;
     // stage the member list and both descriptors in pinned memory; it is not
     // reused before the stream synchronises at the end of the next round block
@@ -2034,14 +2037,8 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
 
   auto t0 = std::chrono::steady_clock::now();
   // the array keeps the previous call's contents: reset what must start empty
-  CK(cudaMemsetAsync(q.table, 0xFF, (size_t)g->V * WT * 8, 0));
-  CK(cudaMemsetAsync(q.dist, 0xFF, (size_t)g->V * ROW * 4, 0));
-  CK(cudaMemset2DAsync(q.dist + FLAGW, ROW * 4, 0, 4, g->V, 0));
-  if (q.dist_nx != q.dist) {
-    CK(cudaMemsetAsync(q.dist_nx, 0xFF, (size_t)g->V * ROW * 4, 0));
-    CK(cudaMemset2DAsync(q.dist_nx + FLAGW, ROW * 4, 0, 4, g->V, 0));
-  }
-  CK(cudaMemsetAsync(q.dflag, 0, L.qbuf - L.dflag, 0));
+  init_workspace(g, q, (L.qbuf - L.dflag) / 16, 0);
+  g->launches++;
   // grids: every SM filled to the occupancy limit of each kernel
   int bl = 0, bh = 0;
   SmallLaunch small;

@@ -743,11 +743,16 @@ struct RelaxCnt {
 };
 
 // Per-warp shared scratch; a warp uses one member at a time: the headers of
-// its distance items (or of a hub chunk), its bound rows' capped distances,
-// or a DP state's merge tile.
+// its distance items (or of a hub chunk), its bound rows' list and capped
+// distances, or a DP state's merge tile.
+struct LbScratch {
+  uint32_t dl[KMAX][32];  // each lane's capped distances
+  uint32_t v[64];         // live vertices still to evaluate, all of query `slot`
+  uint32_t n, slot;
+};
 union WarpScratch {
   RelaxHdr hdr[32];
-  uint32_t dl[KMAX][32];
+  LbScratch lb;
   MergeTile mg;
 };
 
@@ -1157,6 +1162,10 @@ __device__ void dseed_item(const QDev& q, uint32_t item) {
   if (m == 0 || (uint32_t)(__ffs(m) - 1) != gi) return;
   for (uint32_t sub = m; sub; sub = (sub - 1u) & m) {
     uint32_t s = q.phase == PH_HOP ? ((v << q.k) | sub) * (uint32_t)q.nd : ((v << q.k) | sub);
+    // a seed that its bound rules out is no state (a dead vertex has none)
+    if (sub != (uint32_t)q.full &&
+        !lb_ok(0u, ld_round(q.lbt + ((size_t)v << q.k) + ((uint32_t)q.full ^ sub)), ld_best(q.ctl)))
+      continue;
     q.table[s] = pack(0u, 0u);
     if (sub == (uint32_t)q.full) {  // v is in every query group: a cost-0 tree
       atomicMin(&q.ctl->best, 0u);
@@ -1222,15 +1231,6 @@ __device__ void tour_warp(const QDev& q, uint32_t lane) {
   __syncwarp();
 }
 
-// Lower-bound table rows: lbt[v][X] = lower_bound_comp(d(v), X) for every
-// subset X (the per-vertex one_label_lb table of the reference,
-// DPQ.cu:174-224, with the tour bounds of CPUNONHOP.h:436-496), saturated to
-// 16 bits, which only lowers a bound.  32 consecutive items, one vertex per
-// lane.  All lanes evaluate the same subset X at a time, so the bound's
-// loops over the groups of X branch alike in every lane and the tour-table
-// reads are one broadcast per warp; each lane packs 8 entries of its row
-// into one 16-byte store.  Items of different
-// queries in one task are handled run by run.
 // lower_bound_comp for a subset X that every lane of the warp evaluates at
 // the same time: the loops run over the groups of X only, and lane `lane`'s
 // capped distances are read from shared memory (sdl[j][lane]), where a
@@ -1271,8 +1271,103 @@ __device__ __forceinline__ uint32_t lower_bound_uniform(const uint32_t (*sdl)[32
   return max(lb0, max(lb1, lb2));
 }
 
+// Lower-bound table rows: lbt[v][X] = lower_bound_comp(d(v), X) for every
+// subset X (the per-vertex one_label_lb table of the reference,
+// DPQ.cu:174-224, with the tour bounds of CPUNONHOP.h:436-496), saturated to
+// 16 bits, which only lowers a bound.  A warp first looks 32 consecutive
+// vertices over and drops the dead ones, those in no tree of cost at most the
+// incumbent:
+//   - a tree through v that reaches every group costs at least the bound of
+//     (v, all groups);
+//   - a vertex that is no member has two branches in a minimal tree: one
+//     reaches the farthest group, another reaches some group, so it costs at
+//     least the largest plus the smallest distance.
+// A dead vertex's row reads "impossible" and no DP state is ever written,
+// flagged or queued at it, so its state table and flags stay uninitialised.
+// The live ones' are filled here (16-byte stores over runs of neighbouring
+// rows), and their bounds are evaluated 32 at a time from a list that carries
+// over from task to task: all lanes evaluate the same subset X, so the bound's
+// loops over the groups of X branch alike in every lane and the tour-table
+// reads are one broadcast per warp.  Issue-bound: the evaluation is some
+// k^2 / 4 table reads per subset and vertex, the look-over one row and one
+// bound.  Measured against bounds for every vertex and a state table filled
+// at admission: six hop-bounded queries on 2^20 vertices 5.5 -> 4.1 ms (their
+// starts had differed by launches alone before), 48 of them in a batch 34.9 ->
+// 27.2 ms, 48 mixed queries on 3M vertices 226 -> 202 ms.
+__device__ __forceinline__ void lb_stage_row(const QDev& q, bool mine, uint32_t v, uint32_t lane,
+                                             uint32_t (*sdl)[32], uint32_t& dmin, uint32_t& dmax) {
+  uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+  if (mine) {
+    const uint4* row = reinterpret_cast<const uint4*>(q.dist + (size_t)v * ROW);
+    a = ld_round(row);
+    b = ld_round(row + 1);
+  }
+  const uint32_t r[KMAX] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
+  dmin = BIG;
+  dmax = 0u;
+#pragma unroll
+  for (int j = 0; j < KMAX; j++) {
+    const uint32_t d = min(r[j], q.cap1);
+    sdl[j][lane] = d;
+    if (j < q.k) {
+      dmin = min(dmin, d);
+      dmax = max(dmax, d);
+    }
+  }
+}
+
+// Bounds of the first `cnt` (at most 32) listed vertices; the rest move up.
+__device__ void lb_eval(const QDev* qd, uint32_t cnt, uint32_t lane, LbScratch& lb) {
+  const QDev& q = qd[lb.slot];
+  const int k = q.k;
+  const uint32_t K2 = 1u << k;
+  const uint32_t* P = q.tour;
+  const uint32_t* T2 = q.tour + (size_t)k * K2 * k;
+  const bool mine = lane < cnt;
+  const uint32_t v = mine ? lb.v[lane] : 0u;
+  uint32_t dmin, dmax;
+  lb_stage_row(q, mine, v, lane, lb.dl, dmin, dmax);
+  __syncwarp();
+  unsigned short* out = q.lbt + ((size_t)v << k);
+  for (uint32_t x0 = 0; x0 < K2; x0 += 8u) {
+    uint32_t pk[4];
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      uint32_t two = 0;
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const uint32_t X = x0 + 2u * h + e;
+        uint32_t bound = 0;
+        if (X != 0u && X < K2) bound = lower_bound_uniform(lb.dl, lane, k, X, P, T2);
+        const uint32_t ent = bound >= BIG ? LB_INF : min(bound, LB_INF - 1u);
+        two |= ent << (16 * e);
+      }
+      pk[h] = two;
+    }
+    if (mine) {
+      if (K2 >= 8u) {
+        *reinterpret_cast<uint4*>(out + x0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      } else {
+        for (uint32_t X = 0; X < K2; X++) out[X] = (unsigned short)(pk[X >> 1] >> (16 * (X & 1u)));
+      }
+    }
+  }
+  const uint32_t left = lb.n - cnt;  // at most 31
+  const uint32_t mv = lane < left ? lb.v[cnt + lane] : 0u;
+  __syncwarp();
+  if (lane < left) lb.v[lane] = mv;
+  if (lane == 0) lb.n = left;
+  __syncwarp();
+}
+
+// What is left on the warp's list, at the end of its tasks (every lane).
+__device__ __forceinline__ void lb_flush(const QDev* qd, uint32_t lane, LbScratch& lb) {
+  __syncwarp();
+  if (lb.n) lb_eval(qd, lb.n, lane, lb);
+}
+
 __device__ void lbt_rows32(const QDev* qd, const uint32_t* __restrict__ pre, int nslots, uint32_t n_lb,
-                           uint32_t task, uint32_t lane, uint32_t (*sdl)[32]) {
+                           uint32_t task, uint32_t lane, LbScratch& lb) {
   const unsigned FULL = 0xFFFFFFFFu;
   const uint32_t it = task * 32u + lane;
   const bool valid = it < n_lb;
@@ -1287,46 +1382,52 @@ __device__ void lbt_rows32(const QDev* qd, const uint32_t* __restrict__ pre, int
     const QDev& q = qd[si];
     const int k = q.k;
     const uint32_t K2 = 1u << k;
-    const uint32_t* P = q.tour;
-    const uint32_t* T2 = q.tour + (size_t)k * K2 * k;
+    if (lb.n != 0u && lb.slot != si) lb_flush(qd, lane, lb);
     const uint32_t v = mine ? q.lb_off + (it - pre[si]) : 0u;
-    {
-      uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
-      if (mine) {
-        const uint4* row = reinterpret_cast<const uint4*>(q.dist + (size_t)v * ROW);
-        a = ld_round(row);
-        b = ld_round(row + 1);
+    uint32_t dmin, dmax;
+    lb_stage_row(q, mine, v, lane, lb.dl, dmin, dmax);
+    __syncwarp();
+    const uint32_t best = ld_best(q.ctl);
+    bool live = mine && dmax < BIG && (dmin == 0u || dmin + dmax <= best);
+    if (__any_sync(FULL, live)) {
+      const uint32_t all = lower_bound_uniform(lb.dl, lane, k, K2 - 1u, q.tour, q.tour + (size_t)k * K2 * k);
+      live = live && all < BIG && all <= best;
+    }
+    const unsigned mm = __ballot_sync(FULL, mine), am = __ballot_sync(FULL, live);
+    // every row of the run "impossible" (entry 0, the empty set, is 0); the
+    // live ones are written again with their bounds
+    const uint32_t v0 = __shfl_sync(FULL, v, i0), nrow = __popc(mm);
+    if (K2 >= 8u) {
+      uint4* rows = reinterpret_cast<uint4*>(q.lbt + ((size_t)v0 << k));
+      const uint32_t per = K2 / 8u;
+      for (uint32_t i = lane; i < nrow * per; i += 32u)
+        rows[i] = make_uint4((i & (per - 1u)) ? INF32 : 0xFFFF0000u, INF32, INF32, INF32);
+    } else if (mine) {
+      for (uint32_t X = 0; X < K2; X++) q.lbt[((size_t)v << k) + X] = (unsigned short)(X ? LB_INF : 0u);
+    }
+    // state table (and flags, where a vertex's are whole words) of the live rows
+    for (unsigned left = am; left;) {
+      const uint32_t a = (uint32_t)(__ffs(left) - 1);
+      const uint32_t len = __popc(left & ~(left + (1u << a)));  // consecutive set bits from a
+      const uint32_t va = __shfl_sync(FULL, v, a);
+      uint4* tab = reinterpret_cast<uint4*>(q.table + (size_t)va * q.WT);
+      for (uint32_t i = lane; i < len * q.WT / 2u; i += 32u) tab[i] = make_uint4(INF32, INF32, INF32, INF32);
+      if (K2 >= 8u) {
+        uint32_t* fl = q.dflag + (size_t)va * (q.WT / 8u);
+        for (uint32_t i = lane; i < len * q.WT / 8u; i += 32u) fl[i] = 0u;
       }
-      const uint32_t r[KMAX] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
-#pragma unroll
-      for (int j = 0; j < KMAX; j++) sdl[j][lane] = min(r[j], q.cap1);
+      left &= left + (1u << a);
+    }
+    if (am) {
+      if (live) lb.v[lb.n + __popc(am & ((1u << lane) - 1u))] = v;
+      __syncwarp();
+      if (lane == 0) {
+        lb.n += __popc(am);
+        lb.slot = si;
+      }
     }
     __syncwarp();
-    unsigned short* out = q.lbt + ((size_t)v << k);
-    for (uint32_t x0 = 0; x0 < K2; x0 += 8u) {
-      uint32_t pk[4];
-#pragma unroll
-      for (int h = 0; h < 4; h++) {
-        uint32_t two = 0;
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const uint32_t X = x0 + 2u * h + e;
-          uint32_t lb = 0;
-          if (X != 0u && X < K2) lb = lower_bound_uniform(sdl, lane, k, X, P, T2);
-          const uint32_t ent = lb >= BIG ? LB_INF : min(lb, LB_INF - 1u);
-          two |= ent << (16 * e);
-        }
-        pk[h] = two;
-      }
-      if (mine) {
-        if (K2 >= 8u) {
-          *reinterpret_cast<uint4*>(out + x0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        } else {
-          for (uint32_t X = 0; X < K2; X++) out[X] = (unsigned short)(pk[X >> 1] >> (16 * (X & 1u)));
-        }
-      }
-    }
-    __syncwarp();  // the next run reuses the distance stage
+    if (lb.n >= 32u) lb_eval(qd, 32u, lane, lb);
   }
 }
 
@@ -1438,27 +1539,23 @@ __device__ void extract_warp(const QDev& q, const GraphDev& g, uint32_t lane) {
 }
 
 // ---------------------------------------------------------------------------
-// Workspace initialisation of an admitted query, one launch: the state table
-// to INF (all ones), both distance-row buffers to "unknown" (words 0..6 all
-// ones) with no group pending (word 7 zero), and the state flags to zero.
-// 16-byte stores, grid-stride.  (Replaces several memsets per query, one of
-// them a 2D memset over V rows of 4 bytes.)
+// Workspace initialisation of an admitted query, one launch: both
+// distance-row buffers to "unknown" (words 0..6 all ones) with no group pending
+// (word 7 zero), and, for k < 3, the state flags to zero (a vertex's flags are
+// not whole words then).  The state table, up to 7.7 GB at 3M vertices, is not
+// touched: the bound-row pass fills the rows of the vertices that can hold a
+// state.  16-byte stores, grid-stride.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_init_workspace(uint4* __restrict__ table, size_t table_vec,
-                                                        uint4* __restrict__ dist, uint4* __restrict__ dist2,
+__global__ void __launch_bounds__(256) k_init_workspace(uint4* __restrict__ dist, uint4* __restrict__ dist2,
                                                         uint32_t nv, uint4* __restrict__ dflag, size_t dflag_vec) {
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint4 ones = make_uint4(INF32, INF32, INF32, INF32);
   const uint4 tail = make_uint4(INF32, INF32, INF32, 0u);
-  for (size_t i = tid; i < table_vec; i += stride) table[i] = ones;
-  for (size_t v = tid; v < nv; v += stride) {
-    dist[2 * v] = ones;
-    dist[2 * v + 1] = tail;
-    if (dist2 != nullptr) {
-      dist2[2 * v] = ones;
-      dist2[2 * v + 1] = tail;
-    }
+  for (size_t i = tid; i < 2 * (size_t)nv; i += stride) {
+    const uint4 x = (i & 1u) ? tail : ones;
+    dist[i] = x;
+    if (dist2 != nullptr) dist2[i] = x;
   }
   for (size_t i = tid; i < dflag_vec; i += stride) dflag[i] = make_uint4(0u, 0u, 0u, 0u);
 }
@@ -1938,9 +2035,9 @@ __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, 
 // rows (one vertex per lane) and snapshot rows of hop-bounded queries.
 __device__ __forceinline__ void heavy_static_task(const QDev* qd, const uint32_t* pre, const uint32_t* s_lb,
                                                   int nslots, uint32_t ht, uint32_t snap0, uint32_t n_lb,
-                                                  uint32_t n_snap, uint32_t lane, uint32_t (*sdl)[32]) {
+                                                  uint32_t n_snap, uint32_t lane, LbScratch& lb) {
   if (ht < snap0) {
-    lbt_rows32(qd, s_lb, nslots, n_lb, ht, lane, sdl);
+    lbt_rows32(qd, s_lb, nslots, n_lb, ht, lane, lb);
     return;
   }
   // snapshot of a hop-bounded query's distance rows, one row per lane
@@ -2049,14 +2146,16 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
   nslots = min(nslots, (int)sd.nslots);
   __shared__ uint32_t s_lb[MAX_SLOTS + 1];
   __shared__ RelaxHdr s_hub[NW];
-  __shared__ uint32_t s_dl[NW][KMAX][32];  // bound rows: each lane's capped distances
+  __shared__ LbScratch s_lbs[NW];
   __shared__ WarpStat s_ws[NW];
   __shared__ WarpBuf s_wb[NW];
   WarpStat& ws = s_ws[threadIdx.x >> 5];
   WarpBuf& wb = s_wb[threadIdx.x >> 5];
+  LbScratch& lb = s_lbs[threadIdx.x >> 5];
   if (lane == 0) {
     ws_init(ws);
     wb_init(wb);
+    lb.n = 0;
   }
   for (int i = threadIdx.x; i <= nslots; i += blockDim.x) s_lb[i] = __ldcg(pre + T_LB * (MAX_SLOTS + 1) + i);
   __syncthreads();
@@ -2070,8 +2169,9 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     if (task < nbig)
       chunk_task(qd, sd, g, task, lane, &s_hub[threadIdx.x >> 5], ws, wb);
     else
-      heavy_static_task(qd, pre, s_lb, nslots, task - nbig, snap0, n_lb, n_snap, lane, s_dl[threadIdx.x >> 5]);
+      heavy_static_task(qd, pre, s_lb, nslots, task - nbig, snap0, n_lb, n_snap, lane, lb);
   }
+  lb_flush(qd, lane, lb);
   wb_flush(wb, lane);
   if (lane == 0) ws_flush(ws);
 }
@@ -2224,12 +2324,20 @@ __global__ void __launch_bounds__(SMALL_NW * 32, 1)
     }
     const uint32_t ntl = sd.light_tasks, nth = sd.heavy_tasks;
     const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP], snap0 = sd.task_off[T_SNAP];
+    bool lb_used = false;  // the warp's scratch holds a list of bound rows (its light tasks come first)
     for (uint32_t task = warp; task < ntl + nth; task += nwarps) {
+      if (task >= ntl && !lb_used) {
+        lb_used = true;
+        __syncwarp();
+        if (lane == 0) sm.w[wib].lb.n = 0;
+        __syncwarp();
+      }
       if (task < ntl)
         light_task(q, sd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
       else
-        heavy_static_task(q, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].dl);
+        heavy_static_task(q, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].lb);
     }
+    if (lb_used) lb_flush(q, lane, sm.w[wib].lb);
     bool handover = false;
     if (sd.hub_deg != INF32 || sd.grow_chunks != 0u) {
       cluster_barrier();  // the chunk list is complete
@@ -2294,12 +2402,20 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     // light tasks, then the static heavy ones, as one list dealt out over
     // the warps (two lists dealt out one after the other would leave the
     // warps with the heaviest light tasks also the first heavy ones)
+    bool lb_used = false;  // the warp's scratch holds a list of bound rows (its light tasks come first)
     for (uint32_t task = warp; task < ntl + nth; task += nwarps) {
+      if (task >= ntl && !lb_used) {
+        lb_used = true;
+        __syncwarp();
+        if (lane == 0) sm.w[wib].lb.n = 0;
+        __syncwarp();
+      }
       if (task < ntl)
         light_task(qd, sd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
       else
-        heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].dl);
+        heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].lb);
     }
+    if (lb_used) lb_flush(qd, lane, sm.w[wib].lb);
     // phase 1 done in this block: its chunk entries are written.  Rounds
     // that hand out no chunks (every block reads the same flags) skip the
     // grid-wide wait for the others
