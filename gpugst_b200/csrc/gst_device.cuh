@@ -19,9 +19,8 @@
 //   qbuf   u32 [4][cap]        near-in, near-out, far, far-out work lists of state ids
 //   tour   u32 [k][2^k][k] + [k][2^k] + [8][8]  tour tables P, T2 and group distances
 //   lbt    u16 [V][2^k]        lower bound of completing (v, X) to every group
-//   snap   u32 [D-1][V][8]     hop-bounded queries: the distance rows after
-//                               Bellman-Ford round b (b = 1..D-1), i.e. lower
-//                               bounds of the cheapest paths of at most b hops
+//   extra  u32 [n][V][8]       hop-bounded queries: distance rows over paths of
+//                               at most b hops that need a buffer of their own
 #pragma once
 #include <cstdint>
 
@@ -41,12 +40,14 @@ constexpr int DMAX = 7;
 
 // Job state machine (advanced on the device by the control step once per round).
 enum JobState : int32_t { J_FREE = 0, J_INIT, J_SSSP, J_TOUR, J_LB, J_DPSEED, J_DP, J_EXTRACT, J_DONE };
-enum Action : int32_t { A_NONE = 0, A_SSEED, A_WORK, A_SPLIT, A_TOUR, A_LB, A_DSEED, A_EXTRACT };
+enum Action : int32_t { A_NONE = 0, A_SSEED, A_WORK, A_SPLIT, A_TOUR, A_LB, A_DSEED, A_EXTRACT, A_PULL };
 
-// Task types of one round.  Light kernel: split, seeds, tour, extract,
-// distance items and DP states; heavy kernel: the arc chunks the light kernel
-// handed over, then lower-bound table rows.
-enum TaskType : int32_t { T_SPLIT = 0, T_SSEED, T_DSEED, T_TOUR, T_EXTRACT, T_SSSP, T_DP, T_HOP, T_LB, T_SNAP, NT };
+// Task types of one round.  Light kernel: single items (near-far splits and
+// seeds; the query's action says which), tour tables, extraction, distance
+// items, DP states and gathered rows; heavy kernel: the arc chunks the light
+// kernel handed over, then lower-bound table rows and the passes over a round's
+// distance rows.
+enum TaskType : int32_t { T_ITEM = 0, T_TOUR, T_EXTRACT, T_SSSP, T_DP, T_HOP, T_PULL, T_LB, T_ROWS, NT };
 constexpr int MAX_SLOTS = 1024;
 
 // Round-wide work description written by the control step.
@@ -57,8 +58,9 @@ struct RoundDesc {
   uint32_t n_live;        // slots whose job is not finished
   uint32_t n_big;         // arc chunks queued by k_light for k_heavy this round
   // arc chunks: distance items {slot | groups << 16, vertex, first arc, end arc},
-  // DP grow chunks {slot | 1 << 31 (| 1 << 30 hop-bounded), state, first arc,
-  // end arc}; set once by the host (null / 0 disables chunking)
+  // gathered rows {slot | 1 << 29, vertex, first arc, end arc}, DP grow chunks
+  // {slot | 1 << 31 (| 1 << 30 hop-bounded), state, first arc, end arc}; set
+  // once by the host (null / 0 disables chunking)
   uint4* big;
   uint32_t big_cap;
   uint32_t hub_min_deg;   // only items with at least this many arcs under their limit are chunked
@@ -160,23 +162,18 @@ struct alignas(64) QCtl {
   uint32_t pad2[1];
 };
 
-// Per-query descriptor; the host rewrites it before each round.
-struct QDev {
-  unsigned long long* table;
+// The part of a query's descriptor that the control step reads and rewrites.
+struct QRun {
   uint32_t* dist;
-  uint32_t* dflag;
-  uint32_t* qbuf[4];
-  uint32_t* tour;
-  unsigned short* lbt;      // [V][2^k] lower bound per (vertex, uncovered set)
-  const uint32_t* members;  // distance items v*8+j of every query-group member
-  uint32_t* out_edges;      // extraction output (u, v, w) triples
-  QCtl* ctl;
-  uint32_t cap;
+  // Distance rows written by a distance round.  Unbounded queries relax in
+  // place (dist_nx == dist).  Hop-bounded queries run exact (Jacobi)
+  // Bellman-Ford rounds over two row buffers: round b reads dist (the exact
+  // distances over paths of at most b-1 hops) and writes dist_nx, and
+  // the control step swaps the two after the round.
+  uint32_t* dist_nx;
   uint32_t nv;              // number of vertices
   uint32_t n_members;
-  uint32_t max_edges;
-  int32_t k, D, nd, full;
-  uint32_t WT;       // 2^k * nd entries per vertex
+  int32_t D;
   int32_t phase;
   // round fields
   int32_t in_idx, out_idx, far_idx, far2_idx;
@@ -190,17 +187,15 @@ struct QDev {
   uint32_t delta, delta_sssp, delta_dp;
   uint32_t par;      // parity of the items in (or entering) the near list
   uint32_t lb_off;   // bound-table rows (vertices) already computed
-  uint32_t hops;     // distance rounds done (hop-bounded queries stop after D)
-  uint32_t snap_h;   // distance round whose rows k_heavy copies to snap this round (0: none)
-  uint32_t snap_n;   // snapshots taken (rows for b hops: snap[b-1] if b <= snap_n, else dist)
   uint32_t win_items;  // items of the current window's rounds so far
-  uint32_t* snap;    // [D-1][V][8] (hop-bounded queries)
-  // Distance rows written by a distance round.  Unbounded queries relax in
-  // place (dist_nx == dist).  Hop-bounded queries run exact (Jacobi)
-  // Bellman-Ford rounds over two row buffers: round b reads dist (the exact
-  // distances over paths of at most b-1 hops) and writes dist_nx, and
-  // the control step swaps the two after the round.
-  uint32_t* dist_nx;
+  // Hop-bounded distances: rounds 1..push_rounds relax from the vertices that
+  // changed, the later ones gather at the few vertices that still need them
+  // (see pull_task).  list h is qbuf[h]: the members (h = 0) and the vertices
+  // that round h changed.
+  uint32_t hops;     // distance rounds done
+  uint32_t push_rounds;
+  uint32_t n_list[4];
+  uint32_t rows_h;   // distance round whose rows k_heavy goes over this round (0: none)
   // Hop-bounded queries (D >= 2): the round whose exact rows give the
   // incumbent (star_h = floor(D/2): a vertex with every group within star_h
   // hops spans a tree of diameter <= D) and the round whose rows decide
@@ -213,6 +208,36 @@ struct QDev {
   uint32_t ratio_num, ratio_den;
 };
 
+// Per-query descriptor, written by the host at admission.
+struct QDev : QRun {
+  unsigned long long* table;
+  uint32_t* dflag;
+  uint32_t* qbuf[4];
+  uint32_t* tour;
+  unsigned short* lbt;      // [V][2^k] lower bound per (vertex, uncovered set)
+  const uint32_t* members;  // distance items v*8+j of every query-group member
+  uint32_t* out_edges;      // extraction output (u, v, w) triples
+  QCtl* ctl;
+  // Hop-bounded queries: rows[b], b = 1..D, the exact distances over paths of
+  // at most b hops, valid at every vertex within D - b hops of a member (a
+  // state with b hops left has a subtree of at most D - b hops below it, so no
+  // other vertex is ever asked).  The host sets those with a buffer of their
+  // own, the control step the others.
+  uint32_t* rows[DMAX + 1];
+  uint32_t cap;
+  uint32_t max_edges;
+  int32_t k, nd, full;
+  uint32_t WT;       // 2^k * nd entries per vertex
+};
+// Distance rounds of a hop-bounded query that relax from the changed vertices.
+__host__ __device__ inline uint32_t hop_push_rounds(int D) { return D <= 0 ? 0u : (D == 1 ? 1u : (uint32_t)D / 2u); }
+// Row buffers of its own that a hop-bounded query needs: one for each gathered
+// round, and one for each round before the last two relaxed ones (whose rows
+// stay in the two buffers of the exact rounds).
+__host__ __device__ inline uint32_t hop_extra_rows(int D) {
+  const uint32_t P = hop_push_rounds(D);
+  return D <= 0 ? 0u : (uint32_t)D - P + (P > 2u ? P - 2u : 0u);
+}
 static_assert(sizeof(QDev) <= 512, "the allocation-free scratch keeps one 512-byte block for it");
 
 struct GraphDev {

@@ -158,15 +158,6 @@ struct SmallLaunch {
   }
 };
 
-// What must hold before a query's first round: distances unknown with no
-// group pending and, where the bound-row pass does not clear them (k < 3), no
-// state flag set (the flags' span is 256-aligned).
-void init_workspace(const gst_graph* g, const QDev& q, size_t dflag_vec, cudaStream_t s) {
-  k_init_workspace<<<(unsigned)g->num_sms * 8u, 256, 0, s>>>(
-      reinterpret_cast<uint4*>(q.dist), q.dist_nx != q.dist ? reinterpret_cast<uint4*>(q.dist_nx) : nullptr, q.nv,
-      reinterpret_cast<uint4*>(q.dflag), q.k < 3 ? dflag_vec : 0);
-}
-
 // Small rounds that one k_small launch may run: bounds how long a request
 // that arrives meanwhile waits for its admission.
 constexpr uint32_t SMALL_ROUNDS = 64;
@@ -424,7 +415,7 @@ class Arena {
 
 // Workspace layout of one query (see gst_device.cuh).
 struct Layout {
-  size_t table, dist, dist2, dflag, qbuf, tour, lbt, snap, members, edges, total;
+  size_t table, dist, dist2, dflag, qbuf, tour, lbt, extra, members, edges, total;
   uint32_t cap;
 };
 
@@ -452,12 +443,74 @@ Layout layout_for(const gst_graph* g, int k, int D, size_t n_members, uint32_t m
   L.qbuf = o; o = align_up(o + 4 * cap * 4, 256);
   L.tour = o; o = align_up(o + ((size_t)k * (1u << k) * k + (size_t)k * (1u << k) + 64) * 4, 256);
   L.lbt = o; o = align_up(o + (size_t)g->V * (1u << k) * 2, 256);
-  // hop-bounded queries: distance rows after Bellman-Ford rounds 1..D-1
-  L.snap = o; o = align_up(o + (nd >= 3 ? (size_t)(nd - 2) * g->V * ROW * 4 : 0), 256);
+  // hop-bounded queries: distance rows with a buffer of their own
+  L.extra = o; o = align_up(o + (size_t)hop_extra_rows(D) * g->V * ROW * 4, 256);
   L.members = o; o = align_up(o + std::max<size_t>(n_members, 1) * 4, 256);
   L.edges = o; o = align_up(o + (size_t)std::max<uint32_t>(max_edges, 1) * 12, 256);
   L.total = o;
   return L;
+}
+
+// The descriptor of a query with workspace `mem` laid out as L.
+void describe(QDev& q, const gst_graph* g, const gst_tuning& tune, const Layout& L, char* mem, QCtl* ctl, int k, int D,
+              uint32_t n_members, uint32_t max_edges) {
+  memset(&q, 0, sizeof(q));
+  q.table = (unsigned long long*)(mem + L.table);
+  q.dist = (uint32_t*)(mem + L.dist);
+  q.dist_nx = D >= 0 ? (uint32_t*)(mem + L.dist2) : q.dist;
+  q.dflag = (uint32_t*)(mem + L.dflag);
+  for (int b = 0; b < 4; b++) q.qbuf[b] = (uint32_t*)(mem + L.qbuf) + (size_t)b * L.cap;
+  q.tour = (uint32_t*)(mem + L.tour);
+  q.lbt = (unsigned short*)(mem + L.lbt);
+  q.members = (const uint32_t*)(mem + L.members);
+  q.out_edges = (uint32_t*)(mem + L.edges);
+  q.ctl = ctl;
+  q.cap = L.cap;
+  q.nv = g->V;
+  q.n_members = n_members;
+  q.max_edges = max_edges;
+  q.k = k;
+  q.D = D;
+  q.nd = D < 0 ? 1 : D + 1;
+  q.full = (1 << k) - 1;
+  q.WT = (1u << k) * (uint32_t)q.nd;
+  q.phase = PH_SSSP;
+  // hop-bounded queries read an unreached distance as "no path within the
+  // hops left": their distance rounds may only skip what exceeds the
+  // incumbent itself (capping them at cap_pct% of it, with unknown entries
+  // read as "above the cap", admitted 6.6x more DP states on the 3M-vertex
+  // mix through the weaker hop-budget bound)
+  q.cap_num = D >= 0 ? 1u : tune.cap_pct;
+  q.cap_den = D >= 0 ? 1u : 100u;
+  q.star_h = D >= 2 ? (uint32_t)D / 2u : 0u;
+  q.center_h = D >= 2 ? ((uint32_t)D + 1u) / 2u : 0u;
+  // rows with a buffer of their own: the gathered rounds', then those of the
+  // relaxed rounds before the last two
+  q.push_rounds = hop_push_rounds(D);
+  uint32_t* extra = (uint32_t*)(mem + L.extra);
+  for (int b = 1; b <= D; b++)
+    if (b > (int)q.push_rounds || b + 2 <= (int)q.push_rounds) {
+      q.rows[b] = extra;
+      extra += (size_t)g->V * ROW;
+    }
+  q.in_idx = D >= 0 ? 3 : 0;  // (exact rounds keep their lists, from qbuf[0] on)
+  q.out_idx = D >= 0 ? 0 : 1;
+  q.far_idx = 2;
+  q.far2_idx = 3;
+  q.st = J_INIT;
+  q.act = A_NONE;
+  q.delta_sssp = tune.delta_sssp;
+  q.delta_dp = tune.delta_dp;
+  q.ratio_den = RATIO_DEN;
+}
+
+// What must hold before a query's first round: distances unknown with no
+// group pending and, where the bound-row pass does not clear them (k < 3), no
+// state flag set (the flags' span is 256-aligned).
+void init_workspace(const gst_graph* g, const QDev& q, size_t dflag_vec, cudaStream_t s) {
+  k_init_workspace<<<(unsigned)g->num_sms * 8u, 256, 0, s>>>(
+      reinterpret_cast<uint4*>(q.dist), q.dist_nx != q.dist ? reinterpret_cast<uint4*>(q.dist_nx) : nullptr, q.nv,
+      reinterpret_cast<uint4*>(q.dflag), q.k < 3 ? dflag_vec : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -480,10 +533,7 @@ class Runner {
     CK(cudaEventCreateWithFlags(&ev_fin_, cudaEventDisableTiming));
     for (auto& hh : ev_prof_)
       for (auto& e : hh) CK(cudaEventCreate(&e));
-    delta_sssp_ = g_->tune.delta_sssp;
-    delta_dp_ = g_->tune.delta_dp;
-    cap_num_ = g_->tune.cap_pct;
-    cap_den_ = 100;
+    tune_ = g_->tune;
     max_edges_dev_ = env_u32("GSTB_MAX_TREE_EDGES", 1u << 16);
     rounds_per_sync_ = g_->tune.rounds_per_launch;
     trace_ms_ = (double)env_u32("GSTB_TRACE_MS", 0);  // report host iterations slower than this
@@ -680,10 +730,7 @@ class Runner {
 
   // Take the graph's launch parameters (between calls: nothing in flight).
   gst_status apply_tuning() {
-    delta_sssp_ = g_->tune.delta_sssp;
-    delta_dp_ = g_->tune.delta_dp;
-    cap_num_ = g_->tune.cap_pct;
-    cap_den_ = 100;
+    tune_ = g_->tune;
     const uint32_t hub = g_->tune.hub_min_deg, dpw = g_->tune.dp_wmax, ssw = g_->tune.sssp_wmax;
     const uint32_t mst = g_->tune.merge_stage;
     const bool regrid = g_->tune.block_threads != threads_;
@@ -731,47 +778,8 @@ class Runner {
     j->slot = slot;
     Layout L = layout_for(g_, j->k, j->D, j->members.size(), max_edges_dev_, j->cap_req);
     QDev& q = j->qd;
-    memset(&q, 0, sizeof(q));
-    q.table = (unsigned long long*)(j->mem + L.table);
-    q.dist = (uint32_t*)(j->mem + L.dist);
-    q.dist_nx = j->D >= 0 ? (uint32_t*)(j->mem + L.dist2) : q.dist;
-    q.dflag = (uint32_t*)(j->mem + L.dflag);
-    for (int b = 0; b < 4; b++) q.qbuf[b] = (uint32_t*)(j->mem + L.qbuf) + (size_t)b * L.cap;
-    q.tour = (uint32_t*)(j->mem + L.tour);
-    q.lbt = (unsigned short*)(j->mem + L.lbt);
-    q.snap = (uint32_t*)(j->mem + L.snap);
-    q.nv = g_->V;
-    q.members = (const uint32_t*)(j->mem + L.members);
-    q.out_edges = (uint32_t*)(j->mem + L.edges);
-    q.ctl = d_ctl_ + slot;
-    q.cap = L.cap;
-    q.n_members = (uint32_t)j->members.size();
-    q.max_edges = max_edges_dev_;
-    q.k = j->k;
-    q.D = j->D;
-    q.nd = j->nd;
-    q.full = (int)j->full;
-    q.WT = j->WT;
-    q.phase = PH_SSSP;
-    // hop-bounded queries read an unreached distance as "no path within the
-    // hops left": their distance rounds may only skip what exceeds the
-    // incumbent itself (capping them at cap_pct% of it, with unknown entries
-    // read as "above the cap", admitted 6.6x more DP states on the 3M-vertex
-    // mix through the weaker hop-budget bound)
-    q.cap_num = j->D >= 0 ? 1u : cap_num_;
-    q.cap_den = j->D >= 0 ? 1u : cap_den_;
-    q.star_h = j->D >= 2 ? (uint32_t)j->D / 2u : 0u;
-    q.center_h = j->D >= 2 ? ((uint32_t)j->D + 1u) / 2u : 0u;
-    q.in_idx = 0;
-    q.out_idx = 1;
-    q.far_idx = 2;
-    q.far2_idx = 3;
-    q.st = J_INIT;
-    q.act = A_NONE;
-    q.delta_sssp = delta_sssp_;
-    q.delta_dp = delta_dp_;
+    describe(q, g_, tune_, L, j->mem, d_ctl_ + slot, j->k, j->D, (uint32_t)j->members.size(), max_edges_dev_);
     q.ratio_num = j->D < 0 ? j->ratio_num : 0u;
-    q.ratio_den = RATIO_DEN;
     memset(&j->ctl, 0, sizeof(j->ctl));
     j->ctl.best = INF32;
     j->ctl.best_full = INF64;
@@ -1041,16 +1049,16 @@ class Runner {
       cudaEventElapsedTime(&b, ev_prof_[h][3 * r + 1], ev_prof_[h][3 * r + 2]);
       if (h_rdtrace_) {
         // GSTB_TRACE_ROUNDS: one line per profiled round: kernel times and
-        // the work of each task type (k_light: split, distance seed, DP seed,
-        // tour, extract, distance items, DP states, hop states; k_heavy:
-        // bound rows, snapshot rows; plus the arc chunks handed over)
+        // the work of each task type (k_light: split and seed items, tours,
+        // extractions, distance items, DP states, hop states, gathered rows;
+        // k_heavy: bound rows, rows gone over; plus the arc chunks)
         const RoundDesc& d = h_rdtrace_[(size_t)h * 64 + r];
         fprintf(stderr,
-                "gstb round %llu: light %.3f ms heavy %.3f ms | live %u | split %u sseed %u dseed %u tour %u "
-                "extract %u sssp %u (w %u) dp %u hop %u | lb %u snap %u | chunks %u%s\n",
-                (unsigned long long)g_->prof_rounds, a, b, d.n_live, d.items[T_SPLIT], d.items[T_SSEED],
-                d.items[T_DSEED], d.items[T_TOUR], d.items[T_EXTRACT], d.items[T_SSSP], d.sssp_w, d.items[T_DP],
-                d.items[T_HOP], d.items[T_LB], d.items[T_SNAP], d.n_big, d.hub_on ? " (chunking)" : "");
+                "gstb round %llu: light %.3f ms heavy %.3f ms | live %u | items %u tour %u extract %u sssp %u (w %u) "
+                "dp %u hop %u pull %u | lb %u rows %u | chunks %u%s\n",
+                (unsigned long long)g_->prof_rounds, a, b, d.n_live, d.items[T_ITEM], d.items[T_TOUR],
+                d.items[T_EXTRACT], d.items[T_SSSP], d.sssp_w, d.items[T_DP], d.items[T_HOP], d.items[T_PULL],
+                d.items[T_LB], d.items[T_ROWS], d.n_big, d.hub_on ? " (chunking)" : "");
       }
       g_->prof_light_ms += a;
       g_->prof_heavy_ms += b;
@@ -1134,6 +1142,7 @@ class Runner {
   }
 
   gst_graph* g_;
+  gst_tuning tune_{};  // the launch parameters this runner admits queries with
   Arena arena_;
   std::deque<Job*> retry_;  // queries to run again with larger frontier lists
   cudaStream_t stream_ = nullptr;
@@ -1166,8 +1175,8 @@ class Runner {
   cudaEvent_t ev_blk_[2] = {nullptr, nullptr}, ev_fin_ = nullptr;
   cudaEvent_t ev_prof_[2][3 * 64] = {};
   RoundDesc* h_rdtrace_ = nullptr;  // pinned [2][64] round descriptors (GSTB_TRACE_ROUNDS)
-  uint32_t delta_sssp_ = 8, delta_dp_ = 2, max_edges_dev_ = 1u << 16;
-  uint32_t cap_num_ = 1, cap_den_ = 2, rounds_per_sync_ = 6;
+  uint32_t max_edges_dev_ = 1u << 16;
+  uint32_t rounds_per_sync_ = 6;
   cudaEvent_t ev_[2] = {};
   unsigned light_grid_ = 148 * 4, heavy_grid_ = 148 * 2, resident_light_warps_ = 148 * 4 * 8;
   uint32_t threads_ = 256;  // threads per block of the round kernels
@@ -1996,40 +2005,7 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
   char* ws = base + o_ws;
 
   QDev q;
-  memset(&q, 0, sizeof(q));
-  q.table = (unsigned long long*)(ws + L.table);
-  q.dist = (uint32_t*)(ws + L.dist);
-  q.dist_nx = D >= 0 ? (uint32_t*)(ws + L.dist2) : q.dist;
-  q.dflag = (uint32_t*)(ws + L.dflag);
-  for (int b = 0; b < 4; b++) q.qbuf[b] = (uint32_t*)(ws + L.qbuf) + (size_t)b * L.cap;
-  q.tour = (uint32_t*)(ws + L.tour);
-  q.lbt = (unsigned short*)(ws + L.lbt);
-  q.snap = (uint32_t*)(ws + L.snap);
-  q.members = (const uint32_t*)(ws + L.members);
-  q.out_edges = (uint32_t*)(ws + L.edges);
-  q.ctl = d_ctl;
-  q.cap = L.cap;
-  q.nv = g->V;
-  q.n_members = (uint32_t)n_members;
-  q.max_edges = max_edges;
-  q.k = k;
-  q.D = D;
-  q.nd = nd;
-  q.full = (int)((1u << k) - 1u);
-  q.WT = WT;
-  q.phase = PH_SSSP;
-  q.cap_num = D >= 0 ? 1u : g->tune.cap_pct;
-  q.cap_den = D >= 0 ? 1u : 100u;
-  q.star_h = D >= 2 ? (uint32_t)D / 2u : 0u;
-  q.center_h = D >= 2 ? ((uint32_t)D + 1u) / 2u : 0u;
-  q.in_idx = 0;
-  q.out_idx = 1;
-  q.far_idx = 2;
-  q.far2_idx = 3;
-  q.st = J_INIT;
-  q.act = A_NONE;
-  q.delta_sssp = g->tune.delta_sssp;
-  q.delta_dp = g->tune.delta_dp;
+  describe(q, g, g->tune, L, ws, d_ctl, k, D, (uint32_t)n_members, max_edges);
   QCtl c;
   memset(&c, 0, sizeof(c));
   c.best = INF32;

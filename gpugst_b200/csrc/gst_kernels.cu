@@ -228,12 +228,10 @@ __device__ __forceinline__ void push_multi(bool take, uint32_t item, uint32_t wh
 
 // Hop-bounded queries: the largest distance from vertex u to a group of comp
 // over paths of at most b hops (INF32 if one is out of reach), computed by
-// one lane for its own u.  Rows for b hops are the snapshot after round b
-// while snapshots were taken, else the final rows; for b = 0 only u itself
-// counts (distance 0: u is a member).
+// one lane for its own u; for b = 0 only u itself counts (distance 0: u is a
+// member).
 __device__ __forceinline__ uint32_t hop_budget_one(const QDev& q, uint32_t u, uint32_t comp, uint32_t b) {
-  const uint32_t* row = (b >= 1u && b <= q.snap_n) ? q.snap + ((size_t)(b - 1u) * q.nv + u) * ROW
-                                                   : q.dist + (size_t)u * ROW;
+  const uint32_t* row = (b == 0u ? q.dist : q.rows[b]) + (size_t)u * ROW;
   const uint4* r4 = reinterpret_cast<const uint4*>(row);
   const uint4 x = __ldcg(r4), y = __ldcg(r4 + 1);
   const uint32_t r[KMAX] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z};
@@ -1087,6 +1085,173 @@ __device__ void grow_chunk(const QDev* qd, const uint4 item, const GraphDev& g, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Gathered distance rows of hop-bounded queries.  A state at vertex v with b
+// hops left has a subtree of at most D - b hops below it, which holds a member:
+// the rows over b hops are only ever read at vertices within D - b hops of a
+// member, and so are the rows over b - 1 hops at their neighbours.  The first
+// half of the rounds reaches that far anyway and relaxes from the vertices that
+// changed; from round floor(D/2) + 1 on the set shrinks back to the members,
+// and each of its vertices gathers min over its arcs of the neighbour's row over
+// b - 1 hops: plain loads, no atomics, no lists, none of the arcs of the many
+// vertices that no tree can use.  On 3M vertices with D = 4, relaxing in rounds
+// 3 and 4 scanned 83-99% of all 234M arcs each.  Measured against relaxing in
+// all D rounds: 48 queries with D = 2..4 on 2^20 vertices 27.2 -> 4.5 ms, six
+// one at a time 4.1 -> 2.2 ms, 48 mixed queries on 3M vertices 202 -> 117 ms.
+//
+// Four items of the lists 0 .. D - b per warp, 8 lanes each; a vertex with at
+// least hub_min_deg arcs hands all but the first 32 to k_heavy in chunks.
+// ---------------------------------------------------------------------------
+constexpr uint32_t CH_PULL = 1u << 29;  // big-list entry is a chunk of a gathered row
+constexpr uint32_t PULL_LANES = 8;
+constexpr int PULL_U = 4;  // arcs per lane per step
+
+// Item idx of the lists 0, 1, ..: vertex, and the list it is in.
+__device__ __forceinline__ uint32_t list_item(const QDev& q, uint32_t idx, uint32_t& h) {
+  h = 0;
+  while (h < 3u && idx >= q.n_list[h]) idx -= q.n_list[h++];
+  return q.qbuf[h][idx];
+}
+
+__device__ __forceinline__ void load_row(const uint32_t* rows, uint32_t v, uint32_t (&r)[KMAX]) {
+  const uint4* p = reinterpret_cast<const uint4*>(rows + (size_t)v * ROW);
+  const uint4 a = __ldcg(p), b = __ldcg(p + 1);
+  r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w; r[4] = b.x; r[5] = b.y; r[6] = b.z;
+}
+
+// Lower m[] over up to PULL_U arcs a0 + i * stride (< a1) of weight <= lim;
+// returns the arcs taken.
+__device__ __forceinline__ uint32_t pull_arcs(const GraphDev& g, const uint32_t* src, int k, uint32_t a0,
+                                              uint32_t stride, uint32_t a1, uint32_t lim, uint32_t capb,
+                                              uint32_t (&m)[KMAX]) {
+  uint2 arc[PULL_U];
+  bool ok[PULL_U];
+  uint32_t n = 0;
+#pragma unroll
+  for (int u = 0; u < PULL_U; u++) {
+    const uint32_t a = a0 + (uint32_t)u * stride;
+    ok[u] = a < a1;
+    arc[u] = ok[u] ? __ldg(g.adj + a) : make_uint2(0u, 0u);
+  }
+  uint4 x[PULL_U], y[PULL_U];
+#pragma unroll
+  for (int u = 0; u < PULL_U; u++) {
+    x[u] = y[u] = make_uint4(INF32, INF32, INF32, INF32);
+    if (ok[u] && arc[u].y <= lim) {
+      const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)arc[u].x * ROW);
+      x[u] = __ldcg(p);
+      y[u] = __ldcg(p + 1);
+      n++;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < PULL_U; u++) {
+    const uint32_t r[KMAX] = {x[u].x, x[u].y, x[u].z, x[u].w, y[u].x, y[u].y, y[u].z};
+#pragma unroll
+    for (int t = 0; t < KMAX; t++) {
+      const uint32_t d = r[t] + arc[u].y;
+      if (t < k && r[t] != INF32 && d <= capb) m[t] = min(m[t], d);
+    }
+  }
+  return n;
+}
+
+__device__ void pull_task(const QDev* qd, const uint32_t* __restrict__ pre, int nslots, uint32_t total, uint32_t task,
+                          const GraphDev& g, uint32_t lane, WarpStat& ws, const RoundDesc& sd, RoundDesc* rd) {
+  const unsigned FULL = 0xFFFFFFFFu;
+  const uint32_t gl = lane & (PULL_LANES - 1u), g0 = lane - gl;
+  const unsigned gm = ((1u << PULL_LANES) - 1u) << g0;
+  const uint32_t it = task * (32u / PULL_LANES) + g0 / PULL_LANES;
+  uint32_t slot = 0xFFFFFFFFu, arcs = 0;
+  if (it < total) {
+    slot = find_slot(pre, nslots, it);
+    const QDev& q = qd[slot];
+    const int k = q.k;
+    const uint32_t b = q.hops + 1u;
+    const uint32_t* src = q.rows[b - 1u];
+    uint32_t h, m[KMAX];
+    const uint32_t v = list_item(q, it - __ldcg(pre + slot), h);
+    load_row(src, v, m);
+    // a vertex of a list may be in a nearer one too: it is done there
+    bool seen = false;
+    if (h == 1u) {
+#pragma unroll
+      for (int t = 0; t < KMAX; t++) seen = seen || (t < k && m[t] == 0u);
+    } else if (h > 1u) {
+      uint32_t r[KMAX];
+      load_row(q.rows[h - 1u], v, r);
+#pragma unroll
+      for (int t = 0; t < KMAX; t++) seen = seen || (t < k && r[t] != INF32);
+    }
+    if (!seen) {
+      const uint32_t capb = ld_best(q.ctl);  // what exceeds the incumbent is as good as out of reach
+      const uint32_t a0 = __ldg(g.beg + v);
+      uint32_t a1 = arcs_upto(g, v, __ldg(g.beg + v + 1), capb);
+      const uint32_t n = a1 - a0;
+      if (sd.big != nullptr && n >= sd.hub_min_deg && n - HUB_LOCAL >= sd.hub_min_rest) {
+        const uint32_t st0 = a0 + HUB_LOCAL, nch = (a1 - st0 + HUB_CHUNK - 1u) / HUB_CHUNK;
+        uint32_t cb = 0;
+        if (gl == 0u) cb = atomicAdd(&rd->n_big, nch);
+        cb = __shfl_sync(gm, cb, g0);
+        const bool fits = cb + nch <= sd.big_cap;
+        for (uint32_t c = gl; c < nch && cb + c < sd.big_cap; c += PULL_LANES) {
+          const uint32_t s0 = st0 + c * HUB_CHUNK;
+          sd.big[cb + c] = fits ? make_uint4(slot | CH_PULL, v, s0, min(s0 + HUB_CHUNK, a1)) : make_uint4(slot, v, 0u, 0u);
+        }
+        if (fits) a1 = a0 + HUB_LOCAL;
+      }
+      for (uint32_t base = a0; base < a1; base += PULL_LANES * PULL_U)
+        arcs += pull_arcs(g, src, k, base + gl, PULL_LANES, a1, capb, capb, m);
+#pragma unroll
+      for (int t = 0; t < KMAX; t++) m[t] = __reduce_min_sync(gm, m[t]);
+      uint4* out = reinterpret_cast<uint4*>(q.rows[b] + (size_t)v * ROW);
+      if (gl == 0u) out[0] = make_uint4(m[0], m[1], m[2], m[3]);
+      if (gl == 1u) out[1] = make_uint4(m[4], m[5], m[6], 0u);
+    }
+  }
+  __syncwarp();
+  // counters: the 8 lanes of an item, then per query
+#pragma unroll
+  for (uint32_t o = PULL_LANES / 2u; o > 0u; o >>= 1) arcs += __shfl_xor_sync(FULL, arcs, o);
+  for (uint32_t i = 0; i < 32u; i += PULL_LANES) {
+    const uint32_t si = __shfl_sync(FULL, slot, i), a = __shfl_sync(FULL, arcs, i);
+    if (lane == 0 && si != 0xFFFFFFFFu) {
+      ws_add(ws, qd[si].ctl, ST_SSSP, 1u);
+      ws_add(ws, qd[si].ctl, ST_SSSP_ARCS, a);
+    }
+  }
+}
+
+// One chunk of a gathered row (k_heavy, one warp): lowers the row that the
+// vertex's own task wrote.  The arcs ascend in weight, so a chunk whose first
+// arc cannot lower any of the row's distances ends at once.
+__device__ void pull_chunk(const QDev* qd, const uint4 item, const GraphDev& g, uint32_t lane, WarpStat& ws) {
+  const uint32_t slot = item.x & 0xFFFFu, v = item.y;
+  const QDev& q = qd[slot];
+  const int k = q.k;
+  const uint32_t b = q.hops + 1u, capb = ld_best(q.ctl);
+  uint32_t* out = q.rows[b] + (size_t)v * ROW;
+  uint32_t cur[KMAX], m[KMAX], top = 0;
+  load_row(out, 0u, cur);
+#pragma unroll
+  for (int t = 0; t < KMAX; t++) {
+    m[t] = INF32;
+    if (t < k) top = max(top, cur[t]);
+  }
+  const uint32_t lim = min(capb, top == 0u ? 0u : top - 1u);
+  if (__ldg(&g.adj[item.z].y) > lim) return;
+  uint32_t arcs = 0;
+  for (uint32_t base = item.z; base < item.w; base += 32u * PULL_U)
+    arcs += pull_arcs(g, q.rows[b - 1u], k, base + lane, 32u, item.w, lim, capb, m);
+#pragma unroll
+  for (int t = 0; t < KMAX; t++) {
+    const uint32_t x = __reduce_min_sync(0xFFFFFFFFu, m[t]);
+    if (lane == (uint32_t)t && t < k && x < cur[t]) red_min(out + t, x);
+  }
+  const uint32_t a = warp_sum(arcs);
+  if (lane == 0) ws_add(ws, q.ctl, ST_SSSP_ARCS, a);
+}
+
 // Near-far split of one far item: cost in [theta_lo, theta_hi) -> near list;
 // above -> far-out list; below theta_lo it was already expanded at that cost
 // (every new cost is >= the cost of the item that produced it) -> dropped.
@@ -1190,10 +1355,11 @@ __device__ void tour_warp(const QDev& q, uint32_t lane) {
   uint32_t* gd = T2 + (size_t)k * K2;  // [8][8]
   for (uint32_t t = lane; t < 64; t += 32) gd[t] = BIG;
   __syncwarp();
+  const uint32_t* rows = q.D >= 1 ? q.rows[q.D] : q.dist;
   for (uint32_t t = lane; t < q.n_members; t += 32) {
     uint32_t item = q.members[t];
     uint32_t v = item >> 3, i = item & 7u;
-    for (int j = 0; j < k; j++) atomicMin(&gd[i * 8 + j], min(q.dist[(size_t)v * 8 + j], q.cap1));
+    for (int j = 0; j < k; j++) atomicMin(&gd[i * 8 + j], min(rows[(size_t)v * 8 + j], q.cap1));
   }
   __syncwarp();
   // With no feasible tree found yet the distance rounds ran without a cap, so
@@ -1296,13 +1462,37 @@ __device__ __forceinline__ uint32_t lower_bound_uniform(const uint32_t (*sdl)[32
 // 27.2 ms, 48 mixed queries on 3M vertices 226 -> 202 ms.
 __device__ __forceinline__ void lb_stage_row(const QDev& q, bool mine, uint32_t v, uint32_t lane,
                                              uint32_t (*sdl)[32], uint32_t& dmin, uint32_t& dmax) {
-  uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+  uint32_t r[KMAX] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
   if (mine) {
-    const uint4* row = reinterpret_cast<const uint4*>(q.dist + (size_t)v * ROW);
-    a = ld_round(row);
-    b = ld_round(row + 1);
+    load_row(q.dist, v, r);
+    if (q.D >= 0) {
+      // a state at v has at least h hops below it, h the hops from v to the
+      // nearest member: the missing groups are within D - h hops
+      bool member = false, reached = false;
+#pragma unroll
+      for (int t = 0; t < KMAX; t++) {
+        member = member || (t < q.k && r[t] == 0u);
+        reached = reached || (t < q.k && r[t] != INF32);
+      }
+      if (reached && q.D > 0) {
+        uint32_t h = 0;
+        if (!member)
+          for (h = 1; h < q.push_rounds; h++) {
+            load_row(q.rows[h], v, r);
+            bool any = false;
+#pragma unroll
+            for (int t = 0; t < KMAX; t++) any = any || (t < q.k && r[t] != INF32);
+            if (any) break;
+          }
+        if (h < (uint32_t)q.D) {
+          load_row(q.rows[(uint32_t)q.D - h], v, r);
+        } else {
+#pragma unroll
+          for (int t = 0; t < KMAX; t++) r[t] = INF32;  // no hop left, and v is no member
+        }
+      }
+    }
   }
-  const uint32_t r[KMAX] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
   dmin = BIG;
   dmax = 0u;
 #pragma unroll
@@ -1575,7 +1765,16 @@ struct CtlIn {
         overflow(c.overflow), status(c.status), cancel(c.cancel), best_full(c.best_full) {}
 };
 
-__device__ __forceinline__ void absorb(QDev& q, QCtl& c, const CtlIn& in) {
+// After a distance round of a hop-bounded query: the passes over its rows.
+__device__ __forceinline__ void hop_round_over(QRun& q) {
+  if (q.D < 2) return;
+  if (q.hops == q.center_h + 1u) q.center_done = 1u;  // the pass ran during this round
+  if (q.hops < (uint32_t)q.D &&
+      (q.hops + 2u <= q.push_rounds || q.hops == q.star_h || q.hops == q.center_h))
+    q.rows_h = q.hops;
+}
+
+__device__ __forceinline__ void absorb(QRun& q, QDev& qg, QCtl& c, const CtlIn& in) {
   if (in.cancel) {  // the host withdrew the request
     q.st = J_DONE;
     c.final_status = 12;  // GST_CANCELLED
@@ -1589,13 +1788,18 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c, const CtlIn& in) {
     return;
   }
   int t;
-  q.snap_h = 0;  // a snapshot scheduled last round has been copied
+  q.rows_h = 0;  // a pass over rows scheduled last round has run
   switch (q.act) {
     case A_SSEED:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
       q.n_in = in.n_near;
       q.n_far = 0;
       q.st = J_SSSP;
+      if (q.D >= 0) {  // the lists of the exact rounds are kept: list h is qbuf[h]
+        q.in_idx = 0;
+        q.out_idx = 1;
+        q.n_list[0] = in.n_near;
+      }
       break;
     case A_WORK:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
@@ -1604,17 +1808,25 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c, const CtlIn& in) {
       q.par ^= 1u;  // producers of the round flagged the next items with the other parity
       if (q.st == J_SSSP) {
         q.hops++;
-        if (q.dist_nx != q.dist) {  // exact rounds: the rows just written become the current ones
+        if (q.D >= 0) {  // exact rounds: the rows just written become the current ones
           uint32_t* x = q.dist;
           q.dist = q.dist_nx;
           q.dist_nx = x;
+          q.in_idx = (int32_t)q.hops;
+          q.out_idx = (int32_t)min(q.hops + 1u, 3u);
+#pragma unroll
+          for (uint32_t b = 1; b <= 3u; b++)
+            if (b == q.hops) q.n_list[b] = in.n_near;
+          // the last two relaxed rounds' rows stay in the two buffers, earlier
+          // ones are copied to their own while the next round runs
+          if (q.hops + 2u > q.push_rounds) qg.rows[q.hops] = q.dist;
         }
-        if (q.hops == q.center_h + 1u) q.center_done = 1u;  // the pass ran during this round
-        // rows after round b bound the paths of at most b hops: copy them
-        // while the next round runs (a value it lowers in the meantime is
-        // still a valid bound)
-        if (q.D >= 0 && q.hops < (uint32_t)q.D) q.snap_h = q.hops;
+        hop_round_over(q);
       }
+      break;
+    case A_PULL:
+      q.hops++;
+      hop_round_over(q);
       break;
     case A_SPLIT:
       t = q.in_idx; q.in_idx = q.out_idx; q.out_idx = t;
@@ -1652,9 +1864,11 @@ __device__ __forceinline__ void absorb(QDev& q, QCtl& c, const CtlIn& in) {
 // <= D has a vertex with all its vertices within ceil(D/2) hops (a centre of
 // the tree), so when the exact rows of that many hops showed no vertex with
 // every group in reach, the query has no solution.
-__device__ __forceinline__ void hop_rounds_done(QDev& q, QCtl& c, const CtlIn& in) {
+__device__ __forceinline__ void hop_rounds_done(QRun& q, QDev& qg, QCtl& c, const CtlIn& in) {
   if (q.center_h != 0u && q.center_done && in.center == 0u && in.best == INF32) c.infeasible = 1u;
   q.dist_nx = q.dist;
+  // rounds that converged early: the rows over more hops are the last ones
+  for (uint32_t b = q.hops + 1u; b <= (uint32_t)q.D; b++) qg.rows[b] = q.dist;
 }
 
 // Upper end of the near window that starts at lo.
@@ -1673,7 +1887,7 @@ __device__ __forceinline__ void hop_rounds_done(QDev& q, QCtl& c, const CtlIn& i
 // LIGHT_ITEMS items over all live queries, whose rounds are launch and latency;
 // and the rest in one window once an incumbent caps them.
 constexpr uint32_t LIGHT_ITEMS = 16384;
-__device__ __forceinline__ uint32_t window_end(const QDev& q, uint32_t lo, uint32_t best, uint32_t limit) {
+__device__ __forceinline__ uint32_t window_end(const QRun& q, uint32_t lo, uint32_t best, uint32_t limit) {
   uint32_t w = q.delta;
   if (q.phase == PH_SSSP) {
     if (best != INF32 && limit >= lo) w = max(w, limit - lo + 1u);
@@ -1683,7 +1897,7 @@ __device__ __forceinline__ uint32_t window_end(const QDev& q, uint32_t lo, uint3
   return lo + min(w, INF32 - lo);
 }
 
-__device__ __forceinline__ void decide(QDev& q, QCtl& c, const CtlIn& in, uint32_t n_live) {
+__device__ __forceinline__ void decide(QRun& q, QDev& qg, QCtl& c, const CtlIn& in, uint32_t n_live) {
   for (int guard = 0; guard < 8; guard++) {
     switch (q.st) {
       case J_INIT:
@@ -1707,10 +1921,13 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c, const CtlIn& in, uint32
           // final tree has at most D hops, so these are valid lower bounds,
           // and an unreached vertex cannot join a group
           q.cap1 = BIG;
-          q.snap_n = min(q.hops, (uint32_t)q.D - 1u);
-          hop_rounds_done(q, c, in);
+          hop_rounds_done(q, qg, c, in);
           q.st = J_TOUR;
           continue;
+        }
+        if (q.st == J_SSSP && q.D >= 0 && q.hops >= q.push_rounds && (q.hops > q.push_rounds || q.n_in > 0)) {
+          q.act = A_PULL;
+          return;
         }
         if (q.st == J_DP && q.phase == PH_DP && q.ratio_num != 0u && in.best_full != INF64) {
           // Progressive exit (CPUNONHOP.h:730-755, in exact integer
@@ -1752,12 +1969,7 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c, const CtlIn& in, uint32
           return;
         }
         if (q.st == J_SSSP) {
-          // a hop-bounded query whose rounds converged before D: rows for
-          // more hops than the snapshots taken are the final distances
-          if (q.D >= 0) {
-            q.snap_n = min(q.hops, q.D > 0 ? (uint32_t)q.D - 1u : 0u);
-            hop_rounds_done(q, c, in);
-          }
+          if (q.D >= 0) hop_rounds_done(q, qg, c, in);  // its rounds converged before D
           // every distance below theta_hi is exact and every distance <=
           // cap(best) was discovered; unknown ones are >= min(theta_hi, cap+1)
           unsigned long long b1 = in.best == INF32 ? (unsigned long long)INF32 : limit + 1;
@@ -1780,6 +1992,10 @@ __device__ __forceinline__ void decide(QDev& q, QCtl& c, const CtlIn& in, uint32
         q.theta_lo = 0;
         q.delta = q.delta_dp;
         q.theta_hi = window_end(q, 0u, in.best, in.best);
+        q.in_idx = 0;
+        q.out_idx = 1;
+        q.far_idx = 2;
+        q.far2_idx = 3;
         q.n_in = 0;
         q.n_far = 0;
         c.n_near = 0;
@@ -1846,17 +2062,24 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     if (s < nslots) {
       // (a free slot's words are loaded too: its state alone first would put
       // another trip to L2 in front of every live one's)
-      QDev q = qd[s];
+      QDev& qg = qd[s];
+      QRun q = qg;
       QCtl& c = ctl[s];
       const CtlIn in(c);
       if (q.st != J_FREE) atomicMax(&sm.used_hi, (uint32_t)s + 1u);
       if (q.st != J_FREE && q.st != J_DONE) {
-        absorb(q, c, in);
-        if (q.st != J_DONE) decide(q, c, in, sd.n_live);
+        absorb(q, qg, c, in);
+        if (q.st != J_DONE) decide(q, qg, c, in, sd.n_live);
+        const uint32_t n01 = q.n_list[0] + q.n_list[1], n012 = n01 + q.n_list[2];
         switch (q.act) {
-          case A_SSEED: cnt[T_SSEED] = q.n_members; break;
-          case A_DSEED: cnt[T_DSEED] = q.n_members; break;
-          case A_SPLIT: cnt[T_SPLIT] = q.n_far; break;
+          case A_SSEED:
+          case A_DSEED: cnt[T_ITEM] = q.n_members; break;
+          case A_SPLIT: cnt[T_ITEM] = q.n_far; break;
+          case A_PULL: {  // round hops + 1: the lists 0 .. D - (hops + 1)
+            const uint32_t h = (uint32_t)q.D - q.hops - 1u;
+            cnt[T_PULL] = h == 0u ? q.n_list[0] : (h == 1u ? n01 : (h == 2u ? n012 : n012 + q.n_list[3]));
+            break;
+          }
           case A_TOUR: cnt[T_TOUR] = 1; break;
           case A_LB: cnt[T_LB] = min(q.nv - q.lb_off, LB_CHUNK); break;
           case A_EXTRACT: cnt[T_EXTRACT] = 1; break;
@@ -1865,9 +2088,14 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
             break;
           default: break;
         }
-        if (q.snap_h) cnt[T_SNAP] = q.nv;  // copy the distance rows of round snap_h
+        // the pass over the rows of round rows_h: a copy of all of them, or a
+        // look at the vertices within push_rounds hops of a member
+        if (q.rows_h)
+          cnt[T_ROWS] = q.rows_h + 2u <= q.push_rounds
+                            ? q.nv
+                            : (q.push_rounds == 1u ? n01 : (q.push_rounds == 2u ? n012 : n012 + q.n_list[3]));
         if (q.st != J_DONE) atomicAdd(&sm.live_cnt, 1u);
-        qd[s] = q;
+        static_cast<QRun&>(qg) = q;
       }
     }
     // exclusive scan over the chunk's slots, per task type
@@ -1920,9 +2148,10 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     const unsigned long long n_dp = (unsigned long long)sm.carry[T_DP] + sm.carry[T_HOP];
     // A small round: at most SMALL_ARCS arcs a warp of the cluster at the
     // graph's average degree, SMALL_DP states and SMALL_TASKS other tasks
-    const uint32_t n_other = (sm.carry[T_SPLIT] + sm.carry[T_SSEED] + sm.carry[T_DSEED] + 31u) / 32u +
-                             (sm.carry[T_LB] + 31u) / 32u + (sm.carry[T_SNAP] + 31u) / 32u;
-    const bool small = small_warps != 0u && sm.live_cnt != 0u && n_sssp * sd.avg_deg <= SMALL_ARCS * small_warps &&
+    const uint32_t n_other =
+        (sm.carry[T_ITEM] + 31u) / 32u + (sm.carry[T_LB] + 31u) / 32u + (sm.carry[T_ROWS] + 31u) / 32u;
+    const bool small = small_warps != 0u && sm.live_cnt != 0u &&
+                       (n_sssp + sm.carry[T_PULL]) * sd.avg_deg <= SMALL_ARCS * small_warps &&
                        n_dp <= SMALL_DP * small_warps && n_other <= SMALL_TASKS * small_warps;
     sd.small = small ? 1u : 0u;
     const uint32_t lw = small ? small_warps : sd.light_warps;
@@ -1937,7 +2166,7 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
     uint32_t wd = 1;
     while (wd < sd.dp_wmax && n_dp > 2ull * wd * lw) wd <<= 1;
     sd.dp_w = wd;
-    const uint32_t per_task[NT] = {32, 32, 32, 1, 1, w, wd, wd, 32, 32};
+    const uint32_t per_task[NT] = {32, 1, 1, w, wd, wd, 32 / PULL_LANES, 32, 32};
     uint32_t off = 0;
 #pragma unroll
     for (int t = 0; t < NT; t++) {
@@ -1987,15 +2216,15 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
 // k_heavy) and the persistent one (k_rounds) run the same tasks.
 // ---------------------------------------------------------------------------
 
-// Light task `task` (types T_SPLIT .. T_HOP: splits, seeds, tour tables,
-// extraction, distance items, DP states).  s_pre / s_dp / s_hop: the per-slot
+// Light task `task` (types T_ITEM .. T_PULL: splits and seeds, tour tables,
+// extraction, distance items, DP states, gathered rows).  s_pre / s_dp / s_hop: the per-slot
 // prefixes of the distance, DP and hop items, staged in shared memory.
 __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, RoundDesc* rd, const uint32_t* pre,
                                            const uint32_t* s_pre, const uint32_t* s_dp, const uint32_t* s_hop,
                                            int nslots, const GraphDev& g, uint32_t task, uint32_t lane,
                                            WarpStat& ws, WarpBuf& wb, WarpScratch& sc) {
   int t = 0;
-  while (t < T_HOP && task >= sd.task_off[t + 1]) t++;
+  while (t < T_PULL && task >= sd.task_off[t + 1]) t++;
   const uint32_t local = task - sd.task_off[t];
   const uint32_t* P = pre + t * (MAX_SLOTS + 1);
   const uint32_t total = sd.items[t];
@@ -2003,6 +2232,8 @@ __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, 
     sssp_task(qd, s_pre, nslots, total, local, sd.sssp_w, g, lane, ws, sd, rd, sc.hdr, wb);
   } else if (t == T_DP || t == T_HOP) {
     dp_task(qd, t == T_DP ? s_dp : s_hop, nslots, total, local, sd.dp_w, t == T_HOP, g, lane, sd, rd, ws, wb, &sc.mg);
+  } else if (t == T_PULL) {
+    pull_task(qd, P, nslots, total, local, g, lane, ws, sd, rd);
   } else if (t == T_TOUR) {
     tour_warp(qd[find_slot(P, nslots, local)], lane);
   } else if (t == T_EXTRACT) {
@@ -2015,10 +2246,10 @@ __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, 
       slot = find_slot(P, nslots, it);
       const QDev& q = qd[slot];
       const uint32_t idx = it - __ldcg(P + slot);
-      if (t == T_SPLIT) {
+      if (q.act == A_SPLIT) {
         item = q.qbuf[q.far_idx][idx];
         split_item(q, item, toN, toF);
-      } else if (t == T_SSEED) {
+      } else if (q.act == A_SSEED) {
         const uint32_t m = __ldg(q.members + idx);
         item = m >> 3;
         sseed_item(q, m, toN);
@@ -2032,44 +2263,53 @@ __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, 
 }
 
 // Heavy task `ht` that does not depend on the round's light tasks: bound-table
-// rows (one vertex per lane) and snapshot rows of hop-bounded queries.
+// rows (one vertex per lane) and passes over hop-bounded queries' distance rows.
 __device__ __forceinline__ void heavy_static_task(const QDev* qd, const uint32_t* pre, const uint32_t* s_lb,
-                                                  int nslots, uint32_t ht, uint32_t snap0, uint32_t n_lb,
-                                                  uint32_t n_snap, uint32_t lane, LbScratch& lb) {
-  if (ht < snap0) {
+                                                  int nslots, uint32_t ht, uint32_t rows0, uint32_t n_lb,
+                                                  uint32_t n_rows, uint32_t lane, LbScratch& lb) {
+  if (ht < rows0) {
     lbt_rows32(qd, s_lb, nslots, n_lb, ht, lane, lb);
     return;
   }
-  // snapshot of a hop-bounded query's distance rows, one row per lane
-  const uint32_t it = (ht - snap0) * 32u + lane;
-  if (it < n_snap) {
-    const uint32_t* P = pre + T_SNAP * (MAX_SLOTS + 1);
+  // a pass over a hop-bounded query's distance rows, one row per lane
+  const uint32_t it = (ht - rows0) * 32u + lane;
+  if (it < n_rows) {
+    const uint32_t* P = pre + T_ROWS * (MAX_SLOTS + 1);
     const uint32_t slot = find_slot(P, nslots, it);
-    const QDev& qs = qd[slot];
-    const uint32_t v = it - __ldcg(P + slot);
-    const uint4* src = reinterpret_cast<const uint4*>(qs.dist + (size_t)v * ROW);
-    uint4* dst = reinterpret_cast<uint4*>(qs.snap + ((size_t)(qs.snap_h - 1u) * qs.nv + v) * ROW);
-    const uint4 a = __ldcg(src), b = __ldcg(src + 1);
-    dst[0] = a;
-    dst[1] = b;
-    if (qs.snap_h == qs.star_h || qs.snap_h == qs.center_h) {
-      // the rows are the exact distances over paths of at most snap_h hops
-      const uint32_t r[KMAX] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
-      bool all = true;
-      unsigned long long sum = 0;
-#pragma unroll
-      for (int t = 0; t < KMAX; t++)
-        if (t < qs.k) {
-          all = all && r[t] != INF32;
-          sum += r[t];
-        }
-      if (all && qs.snap_h == qs.center_h && __ldca(&qs.ctl->center) == 0u) atomicExch(&qs.ctl->center, 1u);
-      // v joined to every group by its cheapest path of at most star_h
-      // hops: a breadth-first tree from v inside their union has depth <=
-      // star_h, so diameter <= 2 * star_h <= D, at cost <= sum
-      if (all && qs.snap_h == qs.star_h && sum < ld_best(qs.ctl)) atomicMin(&qs.ctl->best, (uint32_t)sum);
+    const QDev& q = qd[slot];
+    const uint32_t h = q.rows_h;
+    if (h + 2u <= q.push_rounds) {  // copy: its buffer is written again two rounds later
+      const uint32_t v = it - __ldcg(P + slot);
+      const uint4* src = reinterpret_cast<const uint4*>(q.dist + (size_t)v * ROW);
+      uint4* dst = reinterpret_cast<uint4*>(q.rows[h] + (size_t)v * ROW);
+      const uint4 a = __ldcg(src), b = __ldcg(src + 1);
+      dst[0] = a;
+      dst[1] = b;
+      return;
     }
+    // the rows are the exact distances over paths of at most h hops
+    uint32_t l, r[KMAX];
+    const uint32_t v = list_item(q, it - __ldcg(P + slot), l);
+    load_row(q.rows[h], v, r);
+    bool all = true;
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int t = 0; t < KMAX; t++)
+      if (t < q.k) {
+        all = all && r[t] != INF32;
+        sum += r[t];
+      }
+    if (all && h == q.center_h && __ldca(&q.ctl->center) == 0u) atomicExch(&q.ctl->center, 1u);
+    // v joined to every group by its cheapest path of at most star_h
+    // hops: a breadth-first tree from v inside their union has depth <=
+    // star_h, so diameter <= 2 * star_h <= D, at cost <= sum
+    if (all && h == q.star_h && sum < ld_best(q.ctl)) atomicMin(&q.ctl->best, (uint32_t)sum);
   }
+}
+
+// Whether the round's light tasks may hand arc chunks over.
+__device__ __forceinline__ bool has_chunks(const RoundDesc& sd) {
+  return sd.big != nullptr && (sd.hub_deg != INF32 || sd.grow_chunks != 0u || sd.items[T_PULL] != 0u);
 }
 
 // Arc chunk `i` that a light task handed over this round (hub vertex of a
@@ -2077,7 +2317,9 @@ __device__ __forceinline__ void heavy_static_task(const QDev* qd, const uint32_t
 __device__ __forceinline__ void chunk_task(const QDev* qd, const RoundDesc& sd, const GraphDev& g, uint32_t i,
                                            uint32_t lane, RelaxHdr* hub, WarpStat& ws, WarpBuf& wb) {
   const uint4 it = __ldcg(sd.big + i);
-  if (it.x & CH_GROW)
+  if (it.x & CH_PULL)
+    pull_chunk(qd, it, g, lane, ws);
+  else if (it.x & CH_GROW)
     grow_chunk(qd, it, g, lane, ws, wb);
   else
     hub_chunk(qd, it, g, lane, hub, ws, wb);
@@ -2129,7 +2371,7 @@ __global__ void __launch_bounds__(NW * 32, GSTB_LIGHT_MIN_BLOCKS * 8 / NW)
 }
 
 // Heavy round kernel: the arc chunks k_light handed over this round, then
-// bound-table rows and snapshot rows.
+// bound-table rows and passes over distance rows.
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, 24 / NW)
     k_heavy(const QDev* __restrict__ qd, RoundDesc* __restrict__ rd, const uint32_t* __restrict__ pre, int nslots,
@@ -2159,8 +2401,8 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
   }
   for (int i = threadIdx.x; i <= nslots; i += blockDim.x) s_lb[i] = __ldcg(pre + T_LB * (MAX_SLOTS + 1) + i);
   __syncthreads();
-  const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP];
-  const uint32_t snap0 = sd.task_off[T_SNAP];  // heavy tasks before the snapshot rows
+  const uint32_t n_lb = sd.items[T_LB], n_rows = sd.items[T_ROWS];
+  const uint32_t rows0 = sd.task_off[T_ROWS];  // heavy tasks before the passes over rows
 #if GSTB_STEAL
   for (uint32_t task = warp; task < ntasks; task = next_task(&rd->next_heavy, nwarps, lane)) {
 #else
@@ -2169,7 +2411,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     if (task < nbig)
       chunk_task(qd, sd, g, task, lane, &s_hub[threadIdx.x >> 5], ws, wb);
     else
-      heavy_static_task(qd, pre, s_lb, nslots, task - nbig, snap0, n_lb, n_snap, lane, lb);
+      heavy_static_task(qd, pre, s_lb, nslots, task - nbig, rows0, n_lb, n_rows, lane, lb);
   }
   lb_flush(qd, lane, lb);
   wb_flush(wb, lane);
@@ -2181,7 +2423,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
 // resident at once).  Block 0 runs the first control step; the last block to
 // finish a round's work runs the next one.  A round is
 //   wait for its control step (epoch) -> light tasks and the static heavy
-//   tasks (bound rows, snapshots), taken by warp striding -> every block done
+//   tasks (bound rows, passes over rows), taken by warp striding -> every block done
 //   with those (phase1: the arc chunks the light tasks handed over are all
 //   written; skipped in rounds that hand out none) -> the chunks -> arrive;
 //   the last block to arrive runs the next control step and publishes it.
@@ -2323,7 +2565,7 @@ __global__ void __launch_bounds__(SMALL_NW * 32, 1)
       __syncthreads();
     }
     const uint32_t ntl = sd.light_tasks, nth = sd.heavy_tasks;
-    const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP], snap0 = sd.task_off[T_SNAP];
+    const uint32_t n_lb = sd.items[T_LB], n_rows = sd.items[T_ROWS], rows0 = sd.task_off[T_ROWS];
     bool lb_used = false;  // the warp's scratch holds a list of bound rows (its light tasks come first)
     for (uint32_t task = warp; task < ntl + nth; task += nwarps) {
       if (task >= ntl && !lb_used) {
@@ -2335,11 +2577,11 @@ __global__ void __launch_bounds__(SMALL_NW * 32, 1)
       if (task < ntl)
         light_task(q, sd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
       else
-        heavy_static_task(q, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].lb);
+        heavy_static_task(q, pre, sm.pre_lb, nslots, task - ntl, rows0, n_lb, n_rows, lane, sm.w[wib].lb);
     }
     if (lb_used) lb_flush(q, lane, sm.w[wib].lb);
     bool handover = false;
-    if (sd.hub_deg != INF32 || sd.grow_chunks != 0u) {
+    if (has_chunks(sd)) {
       cluster_barrier();  // the chunk list is complete
       const uint32_t nbig = sd.big ? min(__ldcg(&rd->n_big), sd.big_cap) : 0u;
       handover = nbig > SMALL_CHUNKS * nwarps;  // too many for the cluster: k_heavy takes them
@@ -2398,7 +2640,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
     }
     __syncthreads();
     const uint32_t ntl = sd.light_tasks, nth = sd.heavy_tasks;
-    const uint32_t n_lb = sd.items[T_LB], n_snap = sd.items[T_SNAP], snap0 = sd.task_off[T_SNAP];
+    const uint32_t n_lb = sd.items[T_LB], n_rows = sd.items[T_ROWS], rows0 = sd.task_off[T_ROWS];
     // light tasks, then the static heavy ones, as one list dealt out over
     // the warps (two lists dealt out one after the other would leave the
     // warps with the heaviest light tasks also the first heavy ones)
@@ -2413,13 +2655,13 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW)
       if (task < ntl)
         light_task(qd, sd, rd, pre, sm.pre_sssp, sm.pre_dp, sm.pre_hop, nslots, g, task, lane, ws, wb, sm.w[wib]);
       else
-        heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, snap0, n_lb, n_snap, lane, sm.w[wib].lb);
+        heavy_static_task(qd, pre, sm.pre_lb, nslots, task - ntl, rows0, n_lb, n_rows, lane, sm.w[wib].lb);
     }
     if (lb_used) lb_flush(qd, lane, sm.w[wib].lb);
     // phase 1 done in this block: its chunk entries are written.  Rounds
     // that hand out no chunks (every block reads the same flags) skip the
     // grid-wide wait for the others
-    if (sd.big != nullptr && (sd.hub_deg != INF32 || sd.grow_chunks != 0u)) {
+    if (has_chunks(sd)) {
       p1++;
       __syncthreads();
       if (threadIdx.x == 0) {
