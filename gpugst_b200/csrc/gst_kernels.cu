@@ -94,7 +94,7 @@ constexpr uint32_t WBUF = 256;
 struct WarpBuf {
   const QDev* q;
   uint32_t nN, nF;
-  uint32_t itN[WBUF], itF[WBUF];
+  uint32_t it[2 * WBUF];  // near-out entries, then far ones (tour_warp's scratch between uses)
 };
 
 __device__ __forceinline__ void wb_init(WarpBuf& b) {  // lane 0
@@ -122,13 +122,13 @@ __device__ __forceinline__ void wb_flush(WarpBuf& b, uint32_t lane) {
     bool ovf = false;
     for (uint32_t i = lane; i < nN; i += 32u) {
       if (bN + i < cap)
-        outN[bN + i] = b.itN[i];
+        outN[bN + i] = b.it[i];
       else
         ovf = true;
     }
     for (uint32_t i = lane; i < nF; i += 32u) {
       if (bF + i < cap)
-        outF[bF + i] = b.itF[i];
+        outF[bF + i] = b.it[WBUF + i];
       else
         ovf = true;
     }
@@ -174,8 +174,8 @@ __device__ __forceinline__ uint32_t append_lists(const bool (&takeN)[U], const b
   uint32_t pN = oN + xN - cN, pF = oF + xF - cF;
 #pragma unroll
   for (int u = 0; u < U; u++) {
-    if (takeN[u]) b.itN[pN++] = item[u];
-    if (takeF[u]) b.itF[pF++] = item[u];
+    if (takeN[u]) b.it[pN++] = item[u];
+    if (takeF[u]) b.it[WBUF + pF++] = item[u];
   }
   __syncwarp();
   if (lane == 0) {
@@ -1342,57 +1342,78 @@ __device__ void dseed_item(const QDev& q, uint32_t item) {
   }
 }
 
-// One warp per query: group-to-group distances gd[i][j] = min over members of
-// group i of the (capped) distance to group j, then the tour tables
+// Tour tables of a query, one warp per starting group i: group-to-group
+// distances gd[a][b] = min over members of group a of the (capped) distance to
+// group b, then
 //   P[i][S][j]  cheapest visiting order of S starting at i, ending at j
 //   T2[i][S]    min_j P[i][S][j]
-// (replaces the host DP of DPQ.cu:409-483 / AllPaths, CPUNONHOP.h:269-386).
-__device__ void tour_warp(const QDev& q, uint32_t lane) {
-  const int k = q.k;
-  const uint32_t K2 = 1u << k;
-  uint32_t* P = q.tour;
-  uint32_t* T2 = q.tour + (size_t)k * K2 * k;
-  uint32_t* gd = T2 + (size_t)k * K2;  // [8][8]
+// for the subsets S that hold i (replaces the host DP of DPQ.cu:409-483 /
+// AllPaths, CPUNONHOP.h:269-386).  Each warp works out gd again (a query has
+// few members; four of a lane's rows are in flight at once) and keeps it and
+// its 2^(k-1) x k table in shared memory: gd[64], Pi[2^(KMAX-1) * KMAX].  A
+// chain of dependent layers; one warp for all of it, through global memory,
+// took 127 us for k = 6 and 366 us for k = 7; this takes 20 and 35.
+constexpr uint32_t TOUR_WORDS = (1u << (KMAX - 1)) * KMAX;
+__device__ __noinline__ void tour_warp(const QDev& q, uint32_t i, uint32_t lane, uint32_t* gd, uint32_t* Pi) {
+  const uint32_t k = (uint32_t)q.k, K2 = 1u << k;
+  const uint32_t* rows = q.D >= 1 ? q.rows[q.D] : q.dist;
   for (uint32_t t = lane; t < 64; t += 32) gd[t] = BIG;
   __syncwarp();
-  const uint32_t* rows = q.D >= 1 ? q.rows[q.D] : q.dist;
-  for (uint32_t t = lane; t < q.n_members; t += 32) {
-    uint32_t item = q.members[t];
-    uint32_t v = item >> 3, i = item & 7u;
-    for (int j = 0; j < k; j++) atomicMin(&gd[i * 8 + j], min(rows[(size_t)v * 8 + j], q.cap1));
+  constexpr int U = 4;
+  for (uint32_t t0 = lane; t0 < q.n_members; t0 += 32 * U) {
+    uint32_t item[U], r[U][KMAX];
+#pragma unroll
+    for (int u = 0; u < U; u++) item[u] = t0 + 32 * u < q.n_members ? __ldg(q.members + t0 + 32 * u) : INF32;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (item[u] != INF32) load_row(rows, item[u] >> 3, r[u]);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (item[u] != INF32) {
+#pragma unroll
+        for (int j = 0; j < KMAX; j++)
+          if (j < (int)k) atomicMin(&gd[(item[u] & 7u) * 8u + j], min(r[u][j], q.cap1));
+      }
   }
   __syncwarp();
   // With no feasible tree found yet the distance rounds ran without a cap, so
   // an unreachable pair of groups proves there is no solution at all.
-  if (lane == 0 && ld_cg(&q.ctl->best) == INF32) {
+  if (i == 0u && lane == 0 && ld_cg(&q.ctl->best) == INF32) {
     bool cut = false;
-    for (int i = 0; i < k; i++)
-      for (int j = 0; j < k; j++)
-        if (i != j && __ldcg(&gd[i * 8 + j]) >= BIG) cut = true;
+    for (uint32_t a = 0; a < k; a++)
+      for (uint32_t b = 0; b < k; b++)
+        if (a != b && gd[a * 8 + b] >= BIG) cut = true;
     if (cut) q.ctl->infeasible = 1u;
   }
-  const uint32_t nP = (uint32_t)k * K2 * (uint32_t)k;
-  for (uint32_t t = lane; t < nP; t += 32) P[t] = BIG;
+  // subsets that hold i, numbered by their other groups
+  const uint32_t n = K2 / 2u;
+  auto subset = [&](uint32_t c) { return ((c >> i) << (i + 1u)) | (c & ((1u << i) - 1u)) | (1u << i); };
+  for (uint32_t t = lane; t < n * k; t += 32) Pi[t] = t == i ? 0u : BIG;
   __syncwarp();
-  for (uint32_t i = lane; i < (uint32_t)k; i += 32) P[((size_t)i * K2 + (1u << i)) * k + i] = 0;
-  __syncwarp();
-  for (int size = 2; size <= k; size++) {
-    for (uint32_t t = lane; t < nP; t += 32) {
-      uint32_t l = t % k, S = (t / k) % K2, i = t / (k * K2);
-      if ((uint32_t)__popc(S) != (uint32_t)size || !(S >> i & 1u) || !(S >> l & 1u) || l == i) continue;
-      uint32_t Sp = S ^ (1u << l);
-      uint32_t bestv = BIG;
-      for (int jj = 0; jj < k; jj++)
-        if (Sp >> jj & 1u) bestv = min(bestv, sat_add(P[((size_t)i * K2 + Sp) * k + jj], __ldcg(&gd[jj * 8 + l])));
-      P[t] = bestv;
+  for (uint32_t size = 1; size < k; size++) {  // other groups visited
+    for (uint32_t t = lane; t < n * k; t += 32) {
+      const uint32_t c = t / k, l = t - c * k, S = subset(c);
+      if ((uint32_t)__popc(c) != size || l == i || !(S >> l & 1u)) continue;
+      const uint32_t cp = c ^ (1u << (l < i ? l : l - 1u));
+      uint32_t best = BIG;
+      for (uint32_t m = S ^ (1u << l); m; m &= m - 1u) {
+        const uint32_t j = __ffs(m) - 1;
+        best = min(best, sat_add(Pi[cp * k + j], gd[j * 8u + l]));
+      }
+      Pi[t] = best;
     }
     __syncwarp();
   }
-  for (uint32_t t = lane; t < (uint32_t)k * K2; t += 32) {
-    uint32_t i = t / K2, S = t % K2;
+  uint32_t* P = q.tour + (size_t)i * K2 * k;
+  uint32_t* T2 = q.tour + (size_t)k * K2 * k + (size_t)i * K2;
+  for (uint32_t t = lane; t < n * k; t += 32) {
+    const uint32_t c = t / k;
+    P[subset(c) * k + (t - c * k)] = Pi[t];
+  }
+  for (uint32_t c = lane; c < n; c += 32) {
     uint32_t m = BIG;
-    for (int l = 0; l < k; l++) m = min(m, P[((size_t)i * K2 + S) * k + l]);
-    T2[t] = m;
+    for (uint32_t l = 0; l < k; l++) m = min(m, Pi[c * k + l]);
+    T2[subset(c)] = m;
   }
   __syncwarp();
 }
@@ -1639,11 +1660,35 @@ __device__ uint32_t arc_weight_warp(const GraphDev& g, uint32_t a, uint32_t b, u
   return INF32;
 }
 
-// Follow parent words from the best full state, emitting (u, v, w) edges;
-// qbuf[0] serves as the explicit stack.  Run by one warp: every lane walks
-// the same states (lane 0 alone writes), and the arc weights are looked up
-// by the whole warp.
-__device__ void extract_warp(const QDev& q, const GraphDev& g, uint32_t lane) {
+// Whether the list [lo, hi), sorted by (weight, neighbour), holds an arc to b of
+// weight w: binary search by one lane.
+__device__ __forceinline__ bool has_arc(const GraphDev& g, uint32_t lo, uint32_t hi, uint32_t b, uint32_t w) {
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2u;
+    const uint2 arc = __ldg(g.adj + mid);
+    if (arc.y == w && arc.x == b) return true;
+    if (arc.y < w || (arc.y == w && arc.x < b))
+      lo = mid + 1u;
+    else
+      hi = mid;
+  }
+  return false;
+}
+
+// Follow parent words from the best full state, emitting (u, v, w) edges.  Run
+// by one warp: every lane holds one state still to follow.  A state's subset
+// is non-empty and a merge splits it into two disjoint parts, so at most k
+// lanes are ever busy; each step is one trip to the state table for all of
+// them, where a single walk took one per state.  An edge's weight is the
+// difference of its two states' costs unless the lower one has been lowered
+// since (only possible beyond what the bounds let through): afterwards each
+// lane checks its edges against the graph, by binary search of the endpoint
+// with fewer arcs, and the rare rest is looked up by the whole warp.  A chain
+// of dependent loads; measured on a 2^20-vertex R-MAT graph, whose trees run
+// through hubs: 0.264 -> 0.022 ms for the round with the slowest extraction of
+// a batch.
+__device__ __noinline__ void extract_warp(const QDev& q, const GraphDev& g, uint32_t lane) {
+  const unsigned FULL = 0xFFFFFFFFu;
   QCtl* ctl = q.ctl;
   const unsigned long long bf = __ldcg(&ctl->best_full);
   if (bf == INF64) {
@@ -1653,73 +1698,77 @@ __device__ void extract_warp(const QDev& q, const GraphDev& g, uint32_t lane) {
     }
     return;
   }
-  const int k = q.k, nd = q.nd;
+  const int k = q.k;
   const bool hop = q.phase == PH_HOP;
-  const uint32_t payload = (uint32_t)bf;
-  const uint32_t root = hop ? payload >> 3 : payload;
-  const uint32_t rd = hop ? (payload & 7u) : 0u;
-  uint32_t* stack = q.qbuf[0];
-  uint32_t sp = 0;
-  const uint32_t full = (uint32_t)q.full;
-  if (lane == 0) stack[0] = hop ? ((root << k) | full) * (uint32_t)nd + rd : ((root << k) | full);
-  sp = 1;
-  __syncwarp();
-  uint32_t ne = 0, steps = 0, status = 0;
+  const uint32_t nd = hop ? (uint32_t)q.nd : 1u;
+  const uint32_t payload = (uint32_t)bf, root = hop ? payload >> 3 : payload;
+  uint32_t s = ((root << k) | (uint32_t)q.full) * nd + (hop ? (payload & 7u) : 0u);
+  bool act = lane == 0;
+  uint32_t ne = 0, status = 0, steps = 0;
+  uint32_t edge = INF32, c_edge = 0;  // the edge that led here: its number and its upper state's cost
   const uint32_t max_steps = 4u * g.V + 64u;
-  while (sp > 0) {
-    if (++steps > max_steps || sp + 2 > q.cap) {
+  while (__any_sync(FULL, act)) {
+    const unsigned long long e = act ? __ldcg(q.table + s) : 0ull;
+    const uint32_t cost = (uint32_t)(e >> 32), par = (uint32_t)e, type = par >> 30;
+    const uint32_t d = s % nd, vp = s / nd, v = vp >> k, p = vp & ((1u << k) - 1u);
+    if (act && edge < q.max_edges) q.out_edges[3 * edge + 2] = c_edge - cost;
+    const bool grow = act && type == 1u, merge = act && type == 2u;
+    const uint32_t p1 = par & 0xFFu, p2 = p ^ p1;
+    const bool bad = act && (cost == INF32 || type == 3u || (grow && hop && d == 0u) ||
+                             (merge && (p1 == 0u || p2 == 0u || (p1 & ~p) != 0u)));
+    if (++steps > max_steps || __any_sync(FULL, bad)) {
       status = 2;
       break;
     }
-    const uint32_t s = __ldcg(stack + --sp);
-    __syncwarp();  // every lane has read the top before lane 0 overwrites it
-    const uint32_t d = hop ? s % (uint32_t)nd : 0u;
-    const uint32_t vp = hop ? s / (uint32_t)nd : s;
-    const uint32_t v = vp >> k, p = vp & ((1u << k) - 1u);
-    const unsigned long long e = __ldcg(q.table + s);
-    if ((uint32_t)(e >> 32) == INF32) {
-      status = 2;
-      break;
-    }
-    const uint32_t par = (uint32_t)e;
-    const uint32_t type = par >> 30;
-    if (type == 1u) {
+    const unsigned gm = __ballot_sync(FULL, grow), mm = __ballot_sync(FULL, merge);
+    edge = INF32;
+    uint32_t s2 = 0;
+    if (grow) {
       const uint32_t u = par & 0x3FFFFFFFu;
-      const uint32_t w = arc_weight_warp(g, v, u, lane);
-      if (lane == 0 && ne < q.max_edges) {
-        q.out_edges[3 * ne] = u;
-        q.out_edges[3 * ne + 1] = v;
-        q.out_edges[3 * ne + 2] = w;
+      edge = ne + __popc(gm & ((1u << lane) - 1u));
+      c_edge = cost;
+      if (edge < q.max_edges) {
+        q.out_edges[3 * edge] = u;
+        q.out_edges[3 * edge + 1] = v;
       }
-      ne++;
-      if (hop && d == 0) {
-        status = 2;
-        break;
-      }
-      if (lane == 0) stack[sp] = hop ? ((u << k) | p) * (uint32_t)nd + d - 1 : ((u << k) | p);
-      sp++;
-    } else if (type == 2u) {
-      const uint32_t p1 = par & 0xFFu, p2 = p ^ p1;
-      if (p1 == 0 || p2 == 0 || (p1 & ~p) != 0) {
-        status = 2;
-        break;
-      }
-      if (lane == 0) {
-        if (hop) {
-          const uint32_t d1 = (par >> 8) & 7u, d2 = (par >> 11) & 7u;
-          stack[sp] = ((v << k) | p1) * (uint32_t)nd + d1;
-          stack[sp + 1] = ((v << k) | p2) * (uint32_t)nd + d2;
-        } else {
-          stack[sp] = (v << k) | p1;
-          stack[sp + 1] = (v << k) | p2;
-        }
-      }
-      sp += 2;
-    } else if (type != 0u) {
-      status = 2;
-      break;
+      s = ((u << k) | p) * nd + (hop ? d - 1u : 0u);
+    } else if (merge) {
+      s = ((v << k) | p1) * nd + (hop ? (par >> 8) & 7u : 0u);
+      s2 = ((v << k) | p2) * nd + (hop ? (par >> 11) & 7u : 0u);
     }
-    __syncwarp();  // lane 0's pushes are visible to the next pop
+    ne += __popc(gm);
+    act = grow || merge;
+    // the second parts go to the free lanes, in order
+    const unsigned idle = ~__ballot_sync(FULL, act);
+    const uint32_t r = __popc(idle & ((1u << lane) - 1u));
+    const bool take = !act && r < (uint32_t)__popc(mm);
+    const uint32_t from = take ? __fns(mm, 0, (int)r + 1) : lane;
+    const uint32_t got = __shfl_sync(FULL, s2, (int)from);
+    if (take) {
+      s = got;
+      act = true;
+    }
+  }
+  __syncwarp();
+  if (status == 0) {
+    const uint32_t n = min(ne, q.max_edges);
+    for (uint32_t i0 = 0; i0 < n; i0 += 32u) {
+      const uint32_t i = i0 + lane;
+      bool miss = false;
+      uint32_t a = 0, b = 0;
+      if (i < n) {
+        a = q.out_edges[3 * i];
+        b = q.out_edges[3 * i + 1];
+        const uint32_t w = q.out_edges[3 * i + 2];
+        const uint32_t a0 = __ldg(g.beg + a), a1 = __ldg(g.beg + a + 1), b0 = __ldg(g.beg + b), b1 = __ldg(g.beg + b + 1);
+        miss = a1 - a0 <= b1 - b0 ? !has_arc(g, a0, a1, b, w) : !has_arc(g, b0, b1, a, w);
+      }
+      for (unsigned m = __ballot_sync(FULL, miss); m; m &= m - 1u) {
+        const int l = __ffs(m) - 1;
+        const uint32_t w = arc_weight_warp(g, __shfl_sync(FULL, b, l), __shfl_sync(FULL, a, l), lane);
+        if (lane == (uint32_t)l) q.out_edges[3 * i + 2] = w;
+      }
+    }
   }
   if (lane == 0) {
     ctl->status = status;
@@ -2080,7 +2129,7 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
             cnt[T_PULL] = h == 0u ? q.n_list[0] : (h == 1u ? n01 : (h == 2u ? n012 : n012 + q.n_list[3]));
             break;
           }
-          case A_TOUR: cnt[T_TOUR] = 1; break;
+          case A_TOUR: cnt[T_TOUR] = (uint32_t)qg.k; break;
           case A_LB: cnt[T_LB] = min(q.nv - q.lb_off, LB_CHUNK); break;
           case A_EXTRACT: cnt[T_EXTRACT] = 1; break;
           case A_WORK:
@@ -2235,7 +2284,11 @@ __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, 
   } else if (t == T_PULL) {
     pull_task(qd, P, nslots, total, local, g, lane, ws, sd, rd);
   } else if (t == T_TOUR) {
-    tour_warp(qd[find_slot(P, nslots, local)], lane);
+    // (the tables' scratch: the warp's append buffer, emptied first)
+    static_assert(sizeof(wb.it) >= TOUR_WORDS * 4 && sizeof(WarpScratch) >= 256, "tour scratch");
+    const uint32_t slot = find_slot(P, nslots, local);
+    wb_flush(wb, lane);
+    tour_warp(qd[slot], local - __ldcg(P + slot), lane, reinterpret_cast<uint32_t*>(&sc), wb.it);
   } else if (t == T_EXTRACT) {
     extract_warp(qd[find_slot(P, nslots, local)], g, lane);
   } else {
