@@ -37,6 +37,7 @@ constexpr int FLAGW = 7;       // the pending-flags word of a row
 constexpr uint32_t FAR_SH = 16;  // far-list byte of the flags word
 __device__ __forceinline__ uint32_t near_sh(uint32_t par) { return par * 8u; }  // near-list byte of a parity
 constexpr int DMAX = 7;
+constexpr uint32_t HOST_EDGES = 128;  // edges of a tree that extraction writes to the host itself
 
 // Job state machine (advanced on the device by the control step once per round).
 enum JobState : int32_t { J_FREE = 0, J_INIT, J_SSSP, J_TOUR, J_LB, J_DPSEED, J_DP, J_EXTRACT, J_DONE };
@@ -217,6 +218,7 @@ struct QDev : QRun {
   unsigned short* lbt;      // [V][2^k] lower bound per (vertex, uncovered set)
   const uint32_t* members;  // distance items v*8+j of every query-group member
   uint32_t* out_edges;      // extraction output (u, v, w) triples
+  uint32_t* host_edges;     // ... of trees of at most HOST_EDGES edges, in mapped host memory (null: none)
   QCtl* ctl;
   // Hop-bounded queries: rows[b], b = 1..D, the exact distances over paths of
   // at most b hops, valid at every vertex within D - b hops of a member (a

@@ -39,7 +39,8 @@ const void* light_kernel(int threads);
 const void* heavy_kernel(int threads);
 const void* rounds_kernel(int threads);
 const void* small_kernel(int* threads, size_t* smem);
-__global__ void k_init_workspace(uint4*, uint4*, uint32_t, uint4*, size_t);
+__global__ void k_admit(const unsigned char*, const uint32_t*, QDev*, QCtl*, RoundDesc*);
+__global__ void k_init_workspace(const QDev*);
 }  // namespace gstb
 
 using namespace gstb;
@@ -157,6 +158,9 @@ struct SmallLaunch {
     return cudaLaunchKernelExC(&cfg, fn, args);
   }
 };
+
+// Room for the offsets of the records staged for one block of rounds.
+constexpr size_t OFFSETS_ROOM = MAX_SLOTS * 4 + 64;
 
 // Small rounds that one k_small launch may run: bounds how long a request
 // that arrives meanwhile waits for its admission.
@@ -504,15 +508,6 @@ void describe(QDev& q, const gst_graph* g, const gst_tuning& tune, const Layout&
   q.ratio_den = RATIO_DEN;
 }
 
-// What must hold before a query's first round: distances unknown with no
-// group pending and, where the bound-row pass does not clear them (k < 3), no
-// state flag set (the flags' span is 256-aligned).
-void init_workspace(const gst_graph* g, const QDev& q, size_t dflag_vec, cudaStream_t s) {
-  k_init_workspace<<<(unsigned)g->num_sms * 8u, 256, 0, s>>>(
-      reinterpret_cast<uint4*>(q.dist), q.dist_nx != q.dist ? reinterpret_cast<uint4*>(q.dist_nx) : nullptr, q.nv,
-      reinterpret_cast<uint4*>(q.dflag), q.k < 3 ? dflag_vec : 0);
-}
-
 // ---------------------------------------------------------------------------
 // Round driver.  Queries occupy slots of device-resident descriptors; every
 // round is k_small -> k_light -> k_heavy, all reading their work from device
@@ -529,7 +524,7 @@ class Runner {
     CK(cudaSetDevice(g_->device));
     CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     for (auto& e : ev_) CK(cudaEventCreate(&e));
-    for (auto& e : ev_blk_) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto& e : ev_blk_) CK(cudaEventCreate(&e));
     CK(cudaEventCreateWithFlags(&ev_fin_, cudaEventDisableTiming));
     for (auto& hh : ev_prof_)
       for (auto& e : hh) CK(cudaEventCreate(&e));
@@ -586,8 +581,11 @@ class Runner {
     // pinned staging for admissions (descriptors + member lists) and for the
     // tree read-back of retired jobs: copies from pinned memory stay
     // asynchronous, pageable ones would synchronise the stream each time
-    stage_cap_ = (size_t)env_u32("GSTB_STAGE_MB", 32) << 20;
+    // (each half has room for its list of record offsets besides)
+    stage_cap_ = ((size_t)env_u32("GSTB_STAGE_MB", 32) << 20) + 2 * OFFSETS_ROOM;
     CK(cudaMallocHost(&h_stage_, stage_cap_));
+    CK(cudaMalloc(&d_stage_, stage_cap_));
+    CK(cudaMallocHost(&h_small_edges_, (size_t)max_slots_ * HOST_EDGES * 12));
     edge_stage_cap_ = (size_t)env_u32("GSTB_EDGE_STAGE_MB", 16) << 20;
     CK(cudaMallocHost(&h_edge_stage_, edge_stage_cap_));
     memset(h_qd_, 0, sizeof(QDev));  // the zero descriptor that frees a slot
@@ -645,6 +643,7 @@ class Runner {
   }
 
   void release() {
+    if (stream_) cudaStreamSynchronize(stream_);  // a last block of empty rounds may still run
     for (Job* j : slots_)
       if (j) free_job(j);
     slots_.clear();
@@ -668,6 +667,10 @@ class Runner {
     h_rdtrace_ = nullptr;
     h_one_ = nullptr;
     if (h_stage_) cudaFreeHost(h_stage_);
+    if (d_stage_) cudaFree(d_stage_);
+    if (h_small_edges_) cudaFreeHost(h_small_edges_);
+    d_stage_ = nullptr;
+    h_small_edges_ = nullptr;
     if (h_edge_stage_) cudaFreeHost(h_edge_stage_);
     h_stage_ = nullptr;
     h_edge_stage_ = nullptr;
@@ -765,7 +768,7 @@ class Runner {
     if (n_used_ >= max_slots_) return false;
     const size_t need = align_up(sizeof(QDev), 64) + align_up(sizeof(QCtl), 64) + align_up(j->members.size() * 4, 64);
     const int sh = (int)(next_block_ & 1);  // staging half of the block this job starts in
-    if (stage_off_[sh] + need > stage_cap_ / 2) return false;  // staging full until that block has run
+    if (stage_off_[sh] + need + OFFSETS_ROOM > stage_cap_ / 2) return false;  // full until that block has run
     void* p = arena_.alloc(j->bytes);
     if (p == nullptr) return false;
     int slot = -1;
@@ -780,29 +783,46 @@ class Runner {
     QDev& q = j->qd;
     describe(q, g_, tune_, L, j->mem, d_ctl_ + slot, j->k, j->D, (uint32_t)j->members.size(), max_edges_dev_);
     q.ratio_num = j->D < 0 ? j->ratio_num : 0u;
+    q.host_edges = h_small_edges_ + (size_t)slot * HOST_EDGES * 3;
     memset(&j->ctl, 0, sizeof(j->ctl));
     j->ctl.best = INF32;
     j->ctl.best_full = INF64;
-    init_workspace(g_, q, (L.qbuf - L.dflag) / 16, stream_);
-    g_->launches++;
-    // stage the member list and both descriptors in pinned memory; it is not
-    // reused before the stream synchronises at the end of the next round block
+    // stage the descriptor, the control block and the member list in pinned
+    // memory; it is not reused before the block that runs them has finished
     char* st = h_stage_ + (size_t)sh * (stage_cap_ / 2) + stage_off_[sh];
     memcpy(st, &q, sizeof(QDev));
     char* stc = st + align_up(sizeof(QDev), 64);
     memcpy(stc, &j->ctl, sizeof(QCtl));
     char* stm = stc + align_up(sizeof(QCtl), 64);
     memcpy(stm, j->members.data(), j->members.size() * 4);
+    staged_.push_back((uint32_t)stage_off_[sh]);
     stage_off_[sh] += need;
     j->first_block = next_block_;
-    cudaMemcpyAsync((void*)q.members, stm, j->members.size() * 4, cudaMemcpyHostToDevice, stream_);
-    cudaMemcpyAsync(d_qd_ + slot, st, sizeof(QDev), cudaMemcpyHostToDevice, stream_);
-    cudaMemcpyAsync(d_ctl_ + slot, stc, sizeof(QCtl), cudaMemcpyHostToDevice, stream_);
     slots_[slot] = j;
     n_used_++;
     nslots_hi_ = std::max<uint32_t>(nslots_hi_, (uint32_t)slot + 1);
     j->t_admit = std::chrono::steady_clock::now();
     return true;
+  }
+
+  // Send the queries admitted since the last call to the device: one copy of
+  // their records (and of the list of their offsets) and one launch.
+  gst_status flush_admissions() {
+    if (staged_.empty()) return GST_OK;
+    const int sh = (int)(next_block_ & 1);
+    char* half = h_stage_ + (size_t)sh * (stage_cap_ / 2);
+    const size_t first = staged_.front(), list = stage_off_[sh], bytes = staged_.size() * 4;
+    memcpy(half + list, staged_.data(), bytes);
+    stage_off_[sh] = align_up(list + bytes, 64);
+    unsigned char* dev = d_stage_ + (size_t)sh * (stage_cap_ / 2);
+    CK(cudaMemcpyAsync(dev + first, half + first, list + bytes - first, cudaMemcpyHostToDevice, stream_));
+    const unsigned n = (unsigned)staged_.size();
+    const unsigned bx = std::max(1u, (unsigned)g_->num_sms * 8u / n);
+    k_admit<<<dim3(bx, n), 256, 0, stream_>>>(dev, reinterpret_cast<const uint32_t*>(dev + list), d_qd_, d_ctl_, d_rd_);
+    g_->launches++;
+    staged_.clear();
+    CK(cudaGetLastError());
+    return GST_OK;
   }
 
   void free_job(Job* j) {
@@ -851,7 +871,7 @@ class Runner {
     int64_t inflight = -1;  // id of the block launched but not yet examined
     std::vector<Job*> fin;  // retired jobs whose tree copies are in flight
     std::vector<size_t> fin_off;
-    int fin_half = 0;
+    int fin_half = 0, seen_half = -1;
     using clk = std::chrono::steady_clock;
     auto ms_since = [](clk::time_point a) { return std::chrono::duration<double, std::milli>(clk::now() - a).count(); };
     double sum_admit = 0, sum_launch = 0, sum_fin = 0, sum_blk = 0, sum_all = 0;
@@ -882,6 +902,16 @@ class Runner {
         retry_.pop_front();
       }
       admit_more();
+      // all done: the block launched ahead holds empty rounds only, and need
+      // not be waited for (launch_block does before it uses that half again)
+      if (n_used_ == 0 && fin.empty() && retry_.empty() && !g_->profile) {
+        if (inflight >= 0) unseen_[inflight & 1] = true;
+        break;
+      }
+      {
+        const gst_status fs = flush_admissions();
+        if (fs != GST_OK) return fs;
+      }
       if (trace_ms_ > 0) t_admit = ms_since(t_it);
       int64_t launched = -1;
       if (n_used_ > 0) {
@@ -901,10 +931,15 @@ class Runner {
         if (trace_ms_ > 0) t_blk = ms_since(t_it);
         stage_off_[h] = 0;  // admissions staged for this block have been copied
         if (g_->profile) accumulate_profile(h);
-        gst_status st = detect_done(inflight, fin, fin_off);
+        seen_half = h;
+        bool copies = false;  // trees too large for extraction to write to the host itself
+        gst_status st = detect_done(inflight, fin, fin_off, copies);
         if (st != GST_OK) return st;
         fin_half = h;
-        if (!fin.empty()) CK(cudaEventRecord(ev_fin_, stream_));
+        if (copies)
+          CK(cudaEventRecord(ev_fin_, stream_));
+        else
+          finalize(fin, fin_off, fin_half, on_done);
       }
       if (trace_ms_ > 0) {
         const double t_all = ms_since(t_it);
@@ -923,10 +958,8 @@ class Runner {
       inflight = launched;
       if (inflight < 0 && n_used_ == 0 && fin.empty() && retry_.empty()) break;
     }
-    CK(cudaEventRecord(ev_[1], stream_));
-    CK(cudaEventSynchronize(ev_[1]));
     float ms = 0;
-    CK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
+    if (seen_half >= 0) CK(cudaEventElapsedTime(&ms, ev_[0], ev_blk_[seen_half]));
     last_call_ms_ = ms;
     if (trace_ms_ > 0 && sum_all >= trace_ms_)
       fprintf(stderr,
@@ -963,6 +996,10 @@ class Runner {
 
   gst_status launch_block(uint32_t R) {
     const int h = (int)(next_block_ & 1);
+    if (unseen_[h]) {  // this half's last block was left running at the end of a call
+      CK(cudaEventSynchronize(ev_blk_[h]));
+      unseen_[h] = false;
+    }
     const bool prof = g_->profile;
     blk_persist_[h] = persist_ && !(prof && h_rdtrace_);  // the per-round trace needs separate launches
     if (nslots_hi_ != slot_hi_) {  // the control steps scan the slots in use
@@ -1068,7 +1105,7 @@ class Runner {
 
   // Jobs that block `blk` saw finish: queue their tree copies, free their
   // workspace and slot (all stream-ordered after the block in flight).
-  gst_status detect_done(int64_t blk, std::vector<Job*>& fin, std::vector<size_t>& fin_off) {
+  gst_status detect_done(int64_t blk, std::vector<Job*>& fin, std::vector<size_t>& fin_off, bool& copies) {
     const int h = (int)(blk & 1);
     const QCtl* snap = h_ctl_ + (size_t)h * MAX_SLOTS;
     char* estage = h_edge_stage_ + (size_t)h * (edge_stage_cap_ / 2);
@@ -1089,7 +1126,10 @@ class Runner {
         j->root = j->ctl.root;
         uint32_t ne = std::min(j->ctl.n_edges, max_edges_dev_);
         j->edges.resize((size_t)ne * 3);
-        if (ne) {
+        if (ne && j->ctl.n_edges <= std::min(HOST_EDGES, max_edges_dev_)) {
+          memcpy(j->edges.data(), h_small_edges_ + (size_t)s * HOST_EDGES * 3, (size_t)ne * 12);
+        } else if (ne) {
+          copies = true;
           if (off + (size_t)ne * 12 <= edge_stage_cap_ / 2) {
             CK(cudaMemcpyAsync(estage + off, j->qd.out_edges, (size_t)ne * 12, cudaMemcpyDeviceToHost, stream_));
             my = off;
@@ -1099,9 +1139,10 @@ class Runner {
           }
         }
       }
-      // free the slot: a zeroed descriptor is J_FREE for the control step (pinned
-      // source, so the copy stays asynchronous)
-      CK(cudaMemcpyAsync(d_qd_ + s, h_qd_, sizeof(QDev), cudaMemcpyHostToDevice, stream_));
+      // a finished query's descriptor is never looked at again; one whose
+      // rounds were cut short is cleared (J_FREE; pinned source, so the copy
+      // stays asynchronous)
+      if (!snap[s].done) CK(cudaMemcpyAsync(d_qd_ + s, h_qd_, sizeof(QDev), cudaMemcpyHostToDevice, stream_));
       free_job(j);
       slots_[s] = nullptr;
       n_used_--;
@@ -1162,10 +1203,14 @@ class Runner {
   uint32_t slot_hi_ = 0;       // the slot bound on the device
   SmallLaunch small_;
   char* h_stage_ = nullptr;
+  unsigned char* d_stage_ = nullptr;
+  std::vector<uint32_t> staged_;  // offsets of the records staged and not yet sent
+  uint32_t* h_small_edges_ = nullptr;  // [slot][HOST_EDGES][3], written by extraction
   char* h_edge_stage_ = nullptr;
   size_t stage_cap_ = 0, stage_off_[2] = {0, 0}, edge_stage_cap_ = 0;
   int64_t next_block_ = 0;
   uint32_t blk_slots_[2] = {0, 0}, prof_rounds_[2] = {0, 0};
+  bool unseen_[2] = {false, false};  // the half's last block held empty rounds only and was not waited for
   bool persist_ = false, blk_persist_[2] = {false, false};
   unsigned rounds_grid_ = 0;  // blocks of the persistent launch (0: cooperative launch unavailable)
   PersistCtl* d_pc_ = nullptr;
@@ -1177,7 +1222,7 @@ class Runner {
   RoundDesc* h_rdtrace_ = nullptr;  // pinned [2][64] round descriptors (GSTB_TRACE_ROUNDS)
   uint32_t max_edges_dev_ = 1u << 16;
   uint32_t rounds_per_sync_ = 6;
-  cudaEvent_t ev_[2] = {};
+  cudaEvent_t ev_[1] = {};  // the start of a call
   unsigned light_grid_ = 148 * 4, heavy_grid_ = 148 * 2, resident_light_warps_ = 148 * 4 * 8;
   uint32_t threads_ = 256;  // threads per block of the round kernels
   const void* kl_ = nullptr;
@@ -2012,9 +2057,6 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
   c.best_full = INF64;
 
   auto t0 = std::chrono::steady_clock::now();
-  // the array keeps the previous call's contents: reset what must start empty
-  init_workspace(g, q, (L.qbuf - L.dflag) / 16, 0);
-  g->launches++;
   // grids: every SM filled to the occupancy limit of each kernel
   int bl = 0, bh = 0;
   SmallLaunch small;
@@ -2034,7 +2076,17 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
     rd0.sssp_wmax = g->tune.sssp_wmax;
     rd0.merge_stage = g->tune.merge_stage;
     rd0.avg_deg = avg_degree(g);
-    CK(cudaMemcpy(d_rd, &rd0, sizeof(RoundDesc), cudaMemcpyHostToDevice));
+    rd0.n_live = 1;
+    // descriptor, control block and round description in one copy
+    unsigned char head[1024] = {};
+    static_assert(sizeof(QDev) <= 512 && sizeof(QCtl) <= 256 && sizeof(RoundDesc) <= 256, "laid out in `head`");
+    memcpy(head + o_qd, &q, sizeof(QDev));
+    memcpy(head + o_ctl, &c, sizeof(QCtl));
+    memcpy(head + o_rd, &rd0, sizeof(RoundDesc));
+    CK(cudaMemcpyAsync(base, head, o_pre, cudaMemcpyHostToDevice, 0));
+    // the array keeps the previous call's contents: reset what must start empty
+    k_init_workspace<<<(unsigned)g->num_sms * 8u, 256, 0, 0>>>(d_qd);
+    g->launches++;
   }
   // member items v*8 + j, staged through a fixed host array (calls are
   // serialised, so one array serves them all): one copy per 64K members
@@ -2053,11 +2105,8 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
     }
     if (n) CK(cudaMemcpy((uint32_t*)q.members + off, stage, n * 4, cudaMemcpyHostToDevice));
   }
-  CK(cudaMemcpy(d_qd, &q, sizeof(QDev), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(d_ctl, &c, sizeof(QCtl), cudaMemcpyHostToDevice));
-
   GraphDev gd{g->d_beg, g->d_adj, g->V, g->d_wcut};
-  const uint32_t R = 6;
+  const uint32_t R = 2;  // most rounds are k_small's; what follows the last one is idle launches
   const uint64_t max_rounds = 1ull << 22;
   uint64_t rounds = 0;
   for (;;) {
