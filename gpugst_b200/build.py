@@ -8,7 +8,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgstb.so")
-SOURCES = ["gst_kernels.cu", "gst_engine.cu"]
+SOURCES = ["gst_kernels.cu", "gst_graph.cu", "gst_engine.cu"]
 HEADERS = ["gst_device.cuh", os.path.join("..", "..", "include", "gstb.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

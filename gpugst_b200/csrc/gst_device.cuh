@@ -242,6 +242,8 @@ __host__ __device__ inline uint32_t hop_extra_rows(int D) {
 }
 static_assert(sizeof(QDev) <= 512, "the allocation-free scratch keeps one 512-byte block for it");
 
+constexpr uint32_t SORT_BLOCK = 4096;  // arcs of a list that one block sorts (gst_graph.cu)
+
 struct GraphDev {
   const uint32_t* beg;   // [V+1]
   const uint2* adj;      // [arcs] {neighbour, weight}, each list sorted by (weight, neighbour)

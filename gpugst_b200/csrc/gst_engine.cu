@@ -41,6 +41,12 @@ const void* rounds_kernel(int threads);
 const void* small_kernel(int* threads, size_t* smem);
 __global__ void k_admit(const unsigned char*, const uint32_t*, QDev*, QCtl*, RoundDesc*);
 __global__ void k_init_workspace(const QDev*);
+__global__ void k_pack_arcs(const uint32_t*, const uint32_t*, uint2*, size_t);
+__global__ void k_sort_lists(const uint32_t*, unsigned long long*, uint32_t);
+__global__ void k_sort_pieces(const uint2*, uint32_t, unsigned long long*);
+__global__ void k_merge_runs(const uint2*, const uint32_t*, uint32_t, unsigned long long*, unsigned long long*, uint32_t,
+                             int);
+__global__ void k_weight_index(const uint32_t*, const uint2*, uint32_t*, uint32_t);
 }  // namespace gstb
 
 using namespace gstb;
@@ -161,6 +167,9 @@ struct SmallLaunch {
 
 // Room for the offsets of the records staged for one block of rounds.
 constexpr size_t OFFSETS_ROOM = MAX_SLOTS * 4 + 64;
+
+// Staging that a runner starts with: some 1,500 records of a usual query.
+constexpr size_t STAGE_FIRST = (4u << 20) + 2 * OFFSETS_ROOM;
 
 // Small rounds that one k_small launch may run: bounds how long a request
 // that arrives meanwhile waits for its admission.
@@ -578,16 +587,15 @@ class Runner {
     memset(h_pc_, 0, 4 * sizeof(PersistCtl));
     if (env_u32("GSTB_TRACE_ROUNDS", 0)) CK(cudaMallocHost(&h_rdtrace_, 2 * 64 * sizeof(RoundDesc)));
     *h_one_ = 1u;
-    // pinned staging for admissions (descriptors + member lists) and for the
-    // tree read-back of retired jobs: copies from pinned memory stay
-    // asynchronous, pageable ones would synchronise the stream each time
-    // (each half has room for its list of record offsets besides)
-    stage_cap_ = ((size_t)env_u32("GSTB_STAGE_MB", 32) << 20) + 2 * OFFSETS_ROOM;
-    CK(cudaMallocHost(&h_stage_, stage_cap_));
-    CK(cudaMalloc(&d_stage_, stage_cap_));
+    // pinned staging for admissions (descriptors + member lists): copies from
+    // pinned memory stay asynchronous, pageable ones would synchronise the
+    // stream each time.  Pinning takes 0.4 ms a MB, so it starts small and grows
+    // when a record does not fit; the read-back of large trees gets its buffer
+    // with the first of them (both at full size at once: 21 of the 24 ms of the
+    // first query on a graph)
+    stage_max_ = ((size_t)env_u32("GSTB_STAGE_MB", 32) << 20) + 2 * OFFSETS_ROOM;
+    if (!set_stage(std::min(stage_max_, STAGE_FIRST))) return GST_CUDA_ERROR;
     CK(cudaMallocHost(&h_small_edges_, (size_t)max_slots_ * HOST_EDGES * 12));
-    edge_stage_cap_ = (size_t)env_u32("GSTB_EDGE_STAGE_MB", 16) << 20;
-    CK(cudaMallocHost(&h_edge_stage_, edge_stage_cap_));
     memset(h_qd_, 0, sizeof(QDev));  // the zero descriptor that frees a slot
     slots_.assign(max_slots_, nullptr);
     if (env_u32("GSTB_ROUND_GRAPH", 1)) {
@@ -762,13 +770,44 @@ class Runner {
   }
   size_t live() const { return n_used_; }
 
+  // Staging of `bytes` in all (two halves) in place of what there is; nothing
+  // staged is still to be copied.
+  bool set_stage(size_t bytes) {
+    if (h_stage_) cudaFreeHost(h_stage_);
+    if (d_stage_) cudaFree(d_stage_);
+    h_stage_ = nullptr;
+    d_stage_ = nullptr;
+    stage_cap_ = 0;
+    cudaError_t e = cudaMallocHost(&h_stage_, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&d_stage_, bytes);
+    if (e != cudaSuccess) {
+      last_cuda_error() = e;
+      cudaGetLastError();
+      return false;
+    }
+    stage_cap_ = bytes;
+    return true;
+  }
+
+  // Room for a record of `need` bytes in staging half sh; false: full until
+  // that block has run (or larger than the staging may get).
+  bool stage_room(int sh, size_t need) {
+    if (stage_off_[sh] + need + OFFSETS_ROOM <= stage_cap_ / 2) return true;
+    const size_t want = 2 * align_up(need + OFFSETS_ROOM, 64);
+    if (stage_off_[sh] != 0 || want > stage_max_) return false;
+    // the half is empty, the other one's records are on the device when the
+    // stream is idle
+    if (cudaStreamSynchronize(stream_) != cudaSuccess) return false;
+    return set_stage(std::min(stage_max_, std::max(want, 2 * stage_cap_)));
+  }
+
   // Allocate the workspace, initialise it and install the job in a free
   // slot; false if no slot or no device memory is available.
   bool admit(Job* j) {
     if (n_used_ >= max_slots_) return false;
     const size_t need = align_up(sizeof(QDev), 64) + align_up(sizeof(QCtl), 64) + align_up(j->members.size() * 4, 64);
     const int sh = (int)(next_block_ & 1);  // staging half of the block this job starts in
-    if (stage_off_[sh] + need + OFFSETS_ROOM > stage_cap_ / 2) return false;  // full until that block has run
+    if (!stage_room(sh, need)) return false;
     void* p = arena_.alloc(j->bytes);
     if (p == nullptr) return false;
     int slot = -1;
@@ -1108,7 +1147,6 @@ class Runner {
   gst_status detect_done(int64_t blk, std::vector<Job*>& fin, std::vector<size_t>& fin_off, bool& copies) {
     const int h = (int)(blk & 1);
     const QCtl* snap = h_ctl_ + (size_t)h * MAX_SLOTS;
-    char* estage = h_edge_stage_ + (size_t)h * (edge_stage_cap_ / 2);
     size_t off = 0;
     // a persistent launch whose bounded wait expired left its queries' rounds
     // unfinished: every query of the block that had not finished fails
@@ -1130,6 +1168,14 @@ class Runner {
           memcpy(j->edges.data(), h_small_edges_ + (size_t)s * HOST_EDGES * 3, (size_t)ne * 12);
         } else if (ne) {
           copies = true;
+          if (!h_edge_stage_) {
+            const size_t cap = (size_t)env_u32("GSTB_EDGE_STAGE_MB", 16) << 20;
+            if (cudaMallocHost(&h_edge_stage_, cap) == cudaSuccess)
+              edge_stage_cap_ = cap;
+            else
+              cudaGetLastError();  // (large trees are then copied synchronously)
+          }
+          char* estage = h_edge_stage_ + (size_t)h * (edge_stage_cap_ / 2);
           if (off + (size_t)ne * 12 <= edge_stage_cap_ / 2) {
             CK(cudaMemcpyAsync(estage + off, j->qd.out_edges, (size_t)ne * 12, cudaMemcpyDeviceToHost, stream_));
             my = off;
@@ -1207,7 +1253,7 @@ class Runner {
   std::vector<uint32_t> staged_;  // offsets of the records staged and not yet sent
   uint32_t* h_small_edges_ = nullptr;  // [slot][HOST_EDGES][3], written by extraction
   char* h_edge_stage_ = nullptr;
-  size_t stage_cap_ = 0, stage_off_[2] = {0, 0}, edge_stage_cap_ = 0;
+  size_t stage_cap_ = 0, stage_max_ = 0, stage_off_[2] = {0, 0}, edge_stage_cap_ = 0;
   int64_t next_block_ = 0;
   uint32_t blk_slots_[2] = {0, 0}, prof_rounds_[2] = {0, 0};
   bool unseen_[2] = {false, false};  // the half's last block held empty rounds only and was not waited for
@@ -1280,6 +1326,171 @@ gst_status fill_result(Job* j, gst_result* r) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
+// Graph creation
+// ---------------------------------------------------------------------------
+namespace {
+
+// Validation of a graph's arcs by host threads, started by the constructor:
+// neighbours in range, weights of at least 1, and the 32-bit cost range.
+class ArcCheck {
+ public:
+  ArcCheck(const uint32_t* csr, const int32_t* w, uint32_t V, uint64_t arcs) : w_(w), V_(V), arcs_(arcs) {
+    const unsigned n = arcs < (1u << 16) ? 1u : std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    for (unsigned t = 0; t < n; t++)
+      th_.emplace_back([=]() {
+        const uint64_t a0 = arcs / n * t, a1 = t + 1 == n ? arcs : arcs / n * (t + 1);
+        bool bad = false;
+        int32_t top = 0;
+        for (uint64_t a = a0; a < a1; a++) {
+          bad |= csr[a] >= V || w[a] < 1;
+          top = std::max(top, w[a]);
+        }
+        if (bad) bad_ = true;
+        uint32_t cur = wmax_;
+        while ((uint32_t)top > cur && !wmax_.compare_exchange_weak(cur, (uint32_t)top)) {
+        }
+      });
+  }
+  ~ArcCheck() { join(); }
+
+  bool ok() {
+    join();
+    if (!done_) {
+      done_ = true;
+      // Integer range: every distance and tree cost is summed in 32 bits and the
+      // lower bounds saturate at BIG = 2^30 (a saturated bound reads as
+      // "unreachable").  A shortest path or a tree has at most V-1 edges, so the
+      // V-1 heaviest arcs bound every such cost; the graph is rejected if that
+      // bound can reach 2^30.
+      if (!bad_ && arcs_ && (uint64_t)(V_ - 1) * wmax_ >= (uint64_t)BIG) {
+        std::vector<uint32_t> ws(w_, w_ + arcs_);
+        const size_t m = std::min<size_t>(ws.size(), (size_t)V_ - 1);
+        std::nth_element(ws.begin(), ws.begin() + m, ws.end(), std::greater<uint32_t>());
+        uint64_t heavy = 0;
+        for (size_t i = 0; i < m; i++) heavy += ws[i];
+        if (heavy >= (uint64_t)BIG) bad_ = true;
+      }
+    }
+    return !bad_;
+  }
+
+ private:
+  void join() {
+    for (auto& t : th_) t.join();
+    th_.clear();
+  }
+  const int32_t* w_;
+  uint32_t V_;
+  uint64_t arcs_;
+  std::vector<std::thread> th_;
+  std::atomic<bool> bad_{false};
+  std::atomic<uint32_t> wmax_{0};
+  bool done_ = false;
+};
+
+// Device memory freed at the end of its scope.
+struct DeviceTmp {
+  void* p = nullptr;
+  ~DeviceTmp() {
+    if (p) cudaFree(p);
+  }
+  bool alloc(size_t n) {
+    if (cudaMalloc(&p, std::max<size_t>(n, 1)) == cudaSuccess) return true;
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
+};
+
+// Offsets, weight-sorted adjacency and weight-bucket index of a graph on its
+// device.  The arcs go over in pieces of ARC_PIECE, so the caller's separate
+// arrays never take more device memory than that beside the adjacency.
+constexpr size_t ARC_PIECE = 32u << 20;
+// Arcs of long lists merged together: bounds the merge's buffer (a longer list
+// is merged alone).
+constexpr size_t MERGE_GROUP = 32u << 20;
+
+gst_status build_adjacency(gst_graph* g, const uint32_t* beg, const uint32_t* csr, const int32_t* w, ArcCheck& check) {
+  const uint32_t V = g->V;
+  const uint64_t arcs = g->arcs;
+  if (cudaMalloc(&g->d_beg, (size_t)(V + 1) * 4) != cudaSuccess ||
+      cudaMalloc(&g->d_adj, std::max<size_t>(arcs, 1) * 8) != cudaSuccess ||
+      cudaMalloc(&g->d_wcut, (size_t)V * 8 * 4) != cudaSuccess) {
+    cudaGetLastError();
+    return GST_OOM;
+  }
+  CK(cudaMemcpy(g->d_beg, beg, (size_t)(V + 1) * 4, cudaMemcpyHostToDevice));
+  const unsigned grid = (unsigned)g->num_sms * 8u;
+  if (arcs) {
+    const size_t piece = std::min<size_t>(arcs, ARC_PIECE);
+    DeviceTmp raw;
+    if (!raw.alloc(piece * 8)) return GST_OOM;
+    uint32_t* d_csr = static_cast<uint32_t*>(raw.p);
+    for (size_t a = 0; a < arcs; a += piece) {
+      const size_t n = std::min<size_t>(piece, arcs - a);
+      CK(cudaMemcpy(d_csr, csr + a, n * 4, cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(d_csr + piece, w + a, n * 4, cudaMemcpyHostToDevice));
+      k_pack_arcs<<<grid, 256>>>(d_csr, d_csr + piece, g->d_adj + a, n);
+      CK(cudaGetLastError());
+    }
+    CK(cudaStreamSynchronize(0));
+  }
+  if (!check.ok()) return GST_BAD_INPUT;
+  unsigned long long* adj = reinterpret_cast<unsigned long long*>(g->d_adj);
+  k_sort_lists<<<grid, 256>>>(g->d_beg, adj, V);
+  CK(cudaGetLastError());
+  // what no warp sorts: pieces for the blocks, and the long lists to merge
+  std::vector<uint2> pieces, lists;
+  for (uint32_t v = 0; v < V; v++) {
+    const uint32_t n = beg[v + 1] - beg[v];
+    if (n <= 256u) continue;
+    for (uint32_t a = 0; a < n; a += SORT_BLOCK) pieces.push_back(make_uint2(beg[v] + a, std::min(SORT_BLOCK, n - a)));
+    if (n > SORT_BLOCK) lists.push_back(make_uint2(beg[v], n));
+  }
+  if (!pieces.empty()) {
+    DeviceTmp dp;
+    if (!dp.alloc(pieces.size() * sizeof(uint2))) return GST_OOM;
+    CK(cudaMemcpy(dp.p, pieces.data(), pieces.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    k_sort_pieces<<<(unsigned)std::min<size_t>(pieces.size(), (size_t)g->num_sms * 4), 512>>>(
+        static_cast<const uint2*>(dp.p), (uint32_t)pieces.size(), adj);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(0));
+  }
+  for (size_t l0 = 0; l0 < lists.size();) {
+    std::vector<uint32_t> cum{0};
+    uint32_t longest = 0;
+    size_t l1 = l0;
+    for (; l1 < lists.size() && (l1 == l0 || cum.back() + (size_t)lists[l1].y <= MERGE_GROUP); l1++) {
+      cum.push_back(cum.back() + lists[l1].y);
+      longest = std::max(longest, lists[l1].y);
+    }
+    const size_t n = l1 - l0;
+    DeviceTmp tmp, dl;
+    if (!tmp.alloc((size_t)cum.back() * 8) || !dl.alloc(n * sizeof(uint2) + cum.size() * 4)) return GST_OOM;
+    uint2* d_list = static_cast<uint2*>(dl.p);
+    uint32_t* d_cum = reinterpret_cast<uint32_t*>(d_list + n);
+    CK(cudaMemcpy(d_list, lists.data() + l0, n * sizeof(uint2), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_cum, cum.data(), cum.size() * 4, cudaMemcpyHostToDevice));
+    int to_tmp = 1;
+    uint64_t width = SORT_BLOCK;
+    for (; width < longest || !to_tmp; width *= 2) {  // an even number of passes ends in the adjacency
+      k_merge_runs<<<grid, 256>>>(d_list, d_cum, (uint32_t)n, adj, static_cast<unsigned long long*>(tmp.p),
+                                  (uint32_t)std::min<uint64_t>(width, 1u << 31), to_tmp);
+      CK(cudaGetLastError());
+      to_tmp ^= 1;
+    }
+    CK(cudaStreamSynchronize(0));
+    l0 = l1;
+  }
+  k_weight_index<<<grid, 256>>>(g->d_beg, g->d_adj, g->d_wcut, V);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(0));
+  return GST_OK;
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------
 extern "C" {
@@ -1313,47 +1524,8 @@ gst_status gst_graph_create(const uint32_t* beg_pos, const uint32_t* csr, const 
   if (beg_pos[0] != 0 || beg_pos[V] != arcs) return GST_BAD_INPUT;
   for (uint32_t v = 0; v < V; v++)
     if (beg_pos[v + 1] < beg_pos[v]) return GST_BAD_INPUT;
-  // validate arcs and build the weight-sorted adjacency on the host
-  std::vector<uint2> adj(arcs);
-  bool bad = false;
-  unsigned nth = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  std::vector<std::thread> th;
-  std::atomic<bool> abad{false};
-  for (unsigned t = 0; t < nth; t++) {
-    th.emplace_back([&, t]() {
-      for (uint32_t v = t; v < V; v += nth) {
-        uint32_t a0 = beg_pos[v], a1 = beg_pos[v + 1];
-        for (uint32_t a = a0; a < a1; a++) {
-          if (csr[a] >= V || w[a] < 1) abad = true;
-          adj[a] = make_uint2(csr[a], (uint32_t)w[a]);
-        }
-        std::sort(adj.begin() + a0, adj.begin() + a1, [](const uint2& x, const uint2& y) {
-          return x.y != y.y ? x.y < y.y : x.x < y.x;
-        });
-      }
-    });
-  }
-  for (auto& x : th) x.join();
-  bad = abad;
-  if (bad) return GST_BAD_INPUT;
-  // Integer range: every distance and tree cost is summed in 32 bits and the
-  // lower bounds saturate at BIG = 2^30 (a saturated bound reads as
-  // "unreachable").  A shortest path or a tree has at most V-1 edges, so the
-  // V-1 heaviest arcs bound every such cost; the graph is rejected if that
-  // bound can reach 2^30.
-  if (arcs) {
-    uint32_t wmax = 0;
-    for (uint64_t a = 0; a < arcs; a++) wmax = std::max(wmax, adj[a].y);
-    if ((uint64_t)(V - 1) * wmax >= (uint64_t)BIG) {
-      std::vector<uint32_t> ws(arcs);
-      for (uint64_t a = 0; a < arcs; a++) ws[a] = adj[a].y;
-      const size_t m = std::min<size_t>(ws.size(), (size_t)V - 1);
-      std::nth_element(ws.begin(), ws.begin() + m, ws.end(), std::greater<uint32_t>());
-      uint64_t heavy = 0;
-      for (size_t i = 0; i < m; i++) heavy += ws[i];
-      if (heavy >= (uint64_t)BIG) return GST_BAD_INPUT;
-    }
-  }
+  // the arcs are validated on the host while the device gets its copy
+  ArcCheck check(csr, w, V, arcs);
   gst_graph* g = new gst_graph();
   g->V = V;
   g->arcs = arcs;
@@ -1376,43 +1548,11 @@ gst_status gst_graph_create(const uint32_t* beg_pos, const uint32_t* csr, const 
       g->total_mem = 0;
     }
   }
-  if (cudaMalloc(&g->d_beg, (size_t)(V + 1) * 4) != cudaSuccess ||
-      cudaMalloc(&g->d_adj, std::max<size_t>(arcs, 1) * 8) != cudaSuccess) {
-    cudaGetLastError();
+  const gst_status built = build_adjacency(g, beg_pos, csr, w, check);
+  if (built != GST_OK) {
+    const bool bad = !check.ok();
     gst_graph_destroy(g);
-    return GST_OOM;
-  }
-  if (cudaMemcpy(g->d_beg, beg_pos, (size_t)(V + 1) * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-      (arcs && cudaMemcpy(g->d_adj, adj.data(), arcs * 8, cudaMemcpyHostToDevice) != cudaSuccess)) {
-    gst_graph_destroy(g);
-    return GST_CUDA_ERROR;
-  }
-  {
-    // weight-bucket index: for each vertex the first arc heavier than 2^b
-    std::vector<uint32_t> wc((size_t)V * 8);
-    std::vector<std::thread> tw;
-    for (unsigned t = 0; t < nth; t++) {
-      tw.emplace_back([&, t]() {
-        for (uint32_t v = t; v < V; v += nth) {
-          uint32_t a = beg_pos[v], a1 = beg_pos[v + 1];
-          for (int b = 0; b < 8; b++) {
-            uint32_t th = 1u << b;
-            while (a < a1 && adj[a].y <= th) a++;
-            wc[(size_t)v * 8 + b] = a;
-          }
-        }
-      });
-    }
-    for (auto& x : tw) x.join();
-    if (cudaMalloc(&g->d_wcut, wc.size() * 4) != cudaSuccess) {
-      cudaGetLastError();
-      gst_graph_destroy(g);
-      return GST_OOM;
-    }
-    if (cudaMemcpy(g->d_wcut, wc.data(), wc.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
-      gst_graph_destroy(g);
-      return GST_CUDA_ERROR;
-    }
+    return bad ? GST_BAD_INPUT : built;
   }
   *out = g;
   return GST_OK;

@@ -3,7 +3,8 @@ every hop bound (which rounds relax and which gather, and the buffers their
 rows are kept in), hub vertices around the chunking threshold, every number of
 groups, and batches around the numbers of slots at which the control step and
 the small-round cluster change their ways (8 descriptors staged, 32 slots in
-one warp)."""
+one warp); and adjacency lists around the sizes at which the graph's creation
+sorts them differently (256 and 4096 arcs, and the merges of longer ones)."""
 import numpy as np
 import pytest
 
@@ -71,3 +72,51 @@ def test_batch_sizes(gst_lib, oracle_mod, n, persistent):
     for q, D, r in zip(queries, Ds, res):
         bad += _check(eng, O, g, gr, q, D, r)
     assert not bad, bad[:10]
+
+
+@pytest.mark.parametrize("n", (1, 2, 31, 33, 255, 256, 257, 4095, 4096, 4097, 8192, 8193, 12289, 70001))
+def test_star_of_every_list_size(gst_lib, n):
+    """A star of n leaves with heavy and equal weights: the tree of two leaves
+    costs the sum of their two arcs, so an arc that the sort of the hub's list
+    lost or misplaced shows as a wrong cost."""
+    eng = gst_lib
+    rng = np.random.default_rng(n)
+    w = rng.choice([1, 2, 3, 64, 128, 129, 255, 256, 257, 3000], size=n).astype(np.int32)
+    g = gen.csr_from_edges(n + 1, np.zeros(n, dtype=np.int64), np.arange(1, n + 1), w)
+    # one group a leaf, and one of the hub
+    gr = gen.Groups(np.arange(n + 2, dtype=np.uint64), np.concatenate([np.arange(1, n + 1), [0]]).astype(np.uint32))
+    pairs = [(int(a), int(b)) for a, b in rng.integers(0, n + 1, size=(60, 2)) if a != b]
+    pairs += [(0, n), (n - 1, n), (int(w.argmax()), n), (int(w.argmin()), n)]
+    E = eng.Engine.from_instance(g, gr)
+    res = E.query_batch([np.array(p, dtype=np.uint32) for p in pairs])
+    E.close()
+    cost = np.append(w, 0)
+    for (a, b), r in zip(pairs, res):
+        assert r.status == eng.GST_OK and r.cost == cost[a] + cost[b], (a, b, r.status, r.cost, cost[a] + cost[b])
+        assert sorted(r.edges[:, 2].tolist()) == sorted(int(c) for c in (cost[a], cost[b]) if c)
+
+
+def test_staging_grows_for_large_member_lists(gst_lib, oracle_mod):
+    """Member lists larger than the staging a runner starts with (2 MB a half):
+    it grows for them, alone and behind others, and small queries go on."""
+    eng, O = gst_lib, oracle_mod
+    V = 900_000
+    rng = np.random.default_rng(4)
+    u = np.arange(1, V)
+    g = gen.csr_from_edges(V, u, (u * rng.random(V - 1)).astype(np.int64), rng.integers(1, 9, V - 1).astype(np.int32))
+    big = [np.arange(i, V, 2) for i in range(2)]  # 1.8 MB of members each
+    ptr = np.cumsum([0, len(big[0]), len(big[1]), 1, 1, 1]).astype(np.uint64)
+    gr = gen.Groups(ptr, np.concatenate([*big, [5, 70_000, 899_999]]).astype(np.uint32))
+    E = eng.Engine.from_instance(g, gr)
+    small = np.array([2, 3, 4], dtype=np.uint32)
+    want = O.prunedpp(g, gr, small, 0).cost
+    queries = [small, np.array([0, 1], dtype=np.uint32), small, np.array([0, 1, 2], dtype=np.uint32), small]
+    for batch in (queries, queries[1:2], queries):
+        res = E.query_batch(batch)
+        for q, r in zip(batch, res):
+            assert r.status == eng.GST_OK
+            if len(q) == 3 and q[0] == 2:
+                assert r.cost == want
+            else:
+                assert not O.validate(g, gr, q, -1, r.cost, r.root, r.edges)
+    E.close()
