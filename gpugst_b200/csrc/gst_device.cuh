@@ -248,16 +248,11 @@ struct GraphDev {
   const uint32_t* beg;   // [V+1]
   const uint2* adj;      // [arcs] {neighbour, weight}, each list sorted by (weight, neighbour)
   uint32_t V;
-  const uint32_t* wcut;  // [V][8]: first arc of v with weight > 2^b (b = 0..7), or null
+  // [V][8]: the first arc of v with weight > 2^b (b = 0..6), and in word 7 the
+  // first arc of v: one row holds a vertex's whole range for most limits
+  const uint32_t* wcut;
 };
-
-// Upper bound on the end of the arcs of v whose weight is <= lim (the list is
-// sorted by weight): one load of the bucket index instead of a search.
-__device__ __forceinline__ uint32_t arcs_upto(const GraphDev& g, uint32_t v, uint32_t a1, uint32_t lim) {
-  if (g.wcut == nullptr || lim > 128u) return a1;
-  uint32_t b = lim <= 1u ? 0u : 32u - __clz(lim - 1u);  // smallest b with 2^b >= lim
-  return __ldg(g.wcut + (size_t)v * 8 + b);
-}
+constexpr uint32_t WCUT_MAX = 64;  // largest limit the index bounds
 
 // DP state flags: 4 bits per state, 8 states per word.  Bits 0 and 1 mark
 // "in the near list" for the two round parities, bit 2 "in the far list".
@@ -292,6 +287,50 @@ __device__ __forceinline__ uint32_t ld_cg(const uint32_t* p) { return __ldcg(p);
 // is an upper bound), and it spares the incumbent's L2 sector a read per item.
 __device__ __forceinline__ uint32_t ld_best(const QCtl* c) { return __ldca(&c->best); }
 __device__ __forceinline__ unsigned long long ld_cg(const unsigned long long* p) { return __ldcg(p); }
+
+// A 32-byte row (a distance row, a weight-index row) with one 256-bit load.  An
+// L1 request takes a cycle for each line it touches, so a row a lane read as two
+// 16-byte halves costs a warp 64 cycles where this costs 32.  ld_row reads at L2
+// (rows that other SMs lower); ld_row_nc through the read-only path (data that no
+// launch writes).
+struct Row8 {
+  uint32_t w[8];
+};
+__device__ __forceinline__ Row8 row_of(unsigned long long a, unsigned long long b, unsigned long long c,
+                                       unsigned long long d) {
+  return Row8{{(uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32), (uint32_t)c, (uint32_t)(c >> 32),
+               (uint32_t)d, (uint32_t)(d >> 32)}};
+}
+__device__ __forceinline__ Row8 ld_row(const uint32_t* p) {
+  unsigned long long a, b, c, d;
+  asm volatile("ld.global.cg.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+  return row_of(a, b, c, d);
+}
+__device__ __forceinline__ Row8 ld_row_nc(const uint32_t* p) {
+  unsigned long long a, b, c, d;
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+  return row_of(a, b, c, d);
+}
+
+// Word i of a row that is kept in registers.
+__device__ __forceinline__ uint32_t sel8(const Row8& r, uint32_t i) {
+  const uint32_t a = i & 1u ? r.w[1] : r.w[0], b = i & 1u ? r.w[3] : r.w[2];
+  const uint32_t c = i & 1u ? r.w[5] : r.w[4], d = i & 1u ? r.w[7] : r.w[6];
+  const uint32_t e = i & 2u ? b : a, f = i & 2u ? d : c;
+  return i & 4u ? f : e;
+}
+// Upper bound on the end of the arcs of v whose weight is <= lim (the list is
+// sorted by weight), from v's row of the weight index.
+__device__ __forceinline__ uint32_t arcs_end(const GraphDev& g, uint32_t v, const Row8& cut, uint32_t lim) {
+  if (lim > WCUT_MAX) return __ldg(g.beg + v + 1);
+  return sel8(cut, lim <= 1u ? 0u : 32u - __clz(lim - 1u));  // smallest b with 2^b >= lim
+}
+// The arcs [a0, a1) of v, up to about weight lim.
+__device__ __forceinline__ void arc_range(const GraphDev& g, uint32_t v, uint32_t lim, uint32_t& a0, uint32_t& a1) {
+  const Row8 cut = ld_row_nc(g.wcut + (size_t)v * 8);
+  a0 = cut.w[7];
+  a1 = arcs_end(g, v, cut, lim);
+}
 
 // Software parallel-bit-deposit of the low bits of x into the set bits of mask.
 __device__ __forceinline__ uint32_t pdep(uint32_t x, uint32_t mask) {

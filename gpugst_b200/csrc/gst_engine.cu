@@ -72,7 +72,7 @@ struct gst_graph {
   uint64_t arcs = 0;
   uint32_t* d_beg = nullptr;
   uint2* d_adj = nullptr;
-  uint32_t* d_wcut = nullptr;  // per vertex: first arc with weight > 2^b, b = 0..7
+  uint32_t* d_wcut = nullptr;  // per vertex: weight-bucket index (GraphDev::wcut)
   // group index (host copy; member lists of a query are built on the host).
   // gst_groups_set replaces it under grp_mu held exclusively; every reader
   // (query preparation in all entry points) holds it shared

@@ -115,13 +115,14 @@ __global__ void __launch_bounds__(256) k_merge_runs(const uint2* __restrict__ li
   }
 }
 
-// Weight-bucket index: for each vertex the first arc heavier than 2^b, b = 0..7.
+// Weight-bucket index: for each vertex the first arc heavier than 2^b, b = 0..6,
+// and its first arc.
 __global__ void __launch_bounds__(256) k_weight_index(const uint32_t* __restrict__ beg, const uint2* __restrict__ adj,
                                                       uint32_t* __restrict__ wcut, uint32_t V) {
   const size_t n = (size_t)V * 8;
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const uint32_t v = (uint32_t)(t >> 3), lim = 1u << (t & 7u);
-    uint32_t a = beg[v], b = beg[v + 1];
+    uint32_t a = beg[v], b = (t & 7u) == 7u ? a : beg[v + 1];
     while (a < b) {
       const uint32_t m = a + (b - a) / 2u;
       if (adj[m].y <= lim)

@@ -226,15 +226,29 @@ __device__ __forceinline__ void push_multi(bool take, uint32_t item, uint32_t wh
   }
 }
 
+// Lower bound on the cost of a tree over the groups of S, whatever its vertices:
+// u16 [2^k] after the tour tables (64 words are kept there).
+__device__ __forceinline__ unsigned short* span_table(const QDev& q) {
+  return reinterpret_cast<unsigned short*>(q.tour + (size_t)q.k * q.k * (1u << q.k) + (size_t)q.k * (1u << q.k));
+}
+
+// Largest arc weight worth a grow from a state of cost c that misses the groups
+// of comp (-1: none): whatever the target, a tree over those groups is still to be
+// paid for.  A heavier arc fails the target's own bound, which this spares the
+// scattered read of: 76% of the targets of the 3M-vertex mix failed it.
+__device__ __forceinline__ int64_t grow_limit(const QDev& q, uint32_t comp, uint32_t c, uint32_t best) {
+  const uint32_t s = ld_round(span_table(q) + comp);
+  return s == LB_INF ? -1 : (int64_t)best - (int64_t)c - (int64_t)s;
+}
+
 // Hop-bounded queries: the largest distance from vertex u to a group of comp
 // over paths of at most b hops (INF32 if one is out of reach), computed by
 // one lane for its own u; for b = 0 only u itself counts (distance 0: u is a
 // member).
 __device__ __forceinline__ uint32_t hop_budget_one(const QDev& q, uint32_t u, uint32_t comp, uint32_t b) {
   const uint32_t* row = (b == 0u ? q.dist : q.rows[b]) + (size_t)u * ROW;
-  const uint4* r4 = reinterpret_cast<const uint4*>(row);
-  const uint4 x = __ldcg(r4), y = __ldcg(r4 + 1);
-  const uint32_t r[KMAX] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z};
+  const Row8 rr = ld_row(row);
+  const uint32_t(&r)[8] = rr.w;
   uint32_t mx = 0;
 #pragma unroll
   for (int j = 0; j < KMAX; j++)
@@ -369,9 +383,8 @@ __device__ __forceinline__ bool push_grow_chunks(const RoundDesc& sd, RoundDesc*
 __device__ __forceinline__ void load_dl(const QDev& q, uint32_t v, uint32_t (&dl)[KMAX],
                                         uint32_t& raw_sum_ok, uint32_t comp,
                                         unsigned long long& raw_sum) {
-  const uint4* row = reinterpret_cast<const uint4*>(q.dist + (size_t)v * 8);
-  uint4 a = ld_round(row), b = ld_round(row + 1);
-  uint32_t r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const Row8 row = ld_row(q.dist + (size_t)v * ROW);
+  const uint32_t(&r)[8] = row.w;
   raw_sum = 0;
   raw_sum_ok = 1;
 #pragma unroll
@@ -486,10 +499,11 @@ __device__ void dp_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_t
   // grow, only from states of cost <= best/2 (optimal-tree decomposition,
   // CPUNONHOP.h:820; exact for the unbounded problem); a high-degree vertex
   // grows its first GROW_LOCAL arcs here and hands the rest to k_heavy
-  if (2ull * c <= best) {
-    const uint32_t lim = best - c;
-    const uint32_t a0 = __ldg(g.beg + v);
-    uint32_t a1 = arcs_upto(g, v, __ldg(g.beg + v + 1), lim);
+  const int64_t glim = 2ull * c <= best ? grow_limit(q, comp, c, best) : -1;
+  if (glim > 0) {
+    const uint32_t lim = (uint32_t)glim;
+    uint32_t a0, a1;
+    arc_range(g, v, lim, a0, a1);
     if (sd.grow_chunks && a1 - a0 >= sd.hub_min_deg &&
         push_grow_chunks(sd, rd, slot, false, s, a0 + GROW_LOCAL, a1, lane))
       a1 = a0 + GROW_LOCAL;
@@ -597,10 +611,11 @@ __device__ void hop_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_
   const uint32_t v = vp >> k, p = vp & (K2 - 1u), comp = full ^ p;
   const unsigned short* lbt = q.lbt;
   GrowCnt gc;
-  if (d < (uint32_t)D) {  // grow d -> d+1 (CPUHOP.h:192-206)
-    const uint32_t lim = best - c;
-    const uint32_t a0 = __ldg(g.beg + v);
-    uint32_t a1 = arcs_upto(g, v, __ldg(g.beg + v + 1), lim);
+  const int64_t glim = d < (uint32_t)D ? grow_limit(q, comp, c, best) : -1;
+  if (glim > 0) {  // grow d -> d+1 (CPUHOP.h:192-206)
+    const uint32_t lim = (uint32_t)glim;
+    uint32_t a0, a1;
+    arc_range(g, v, lim, a0, a1);
     if (sd.grow_chunks && a1 - a0 >= sd.hub_min_deg &&
         push_grow_chunks(sd, rd, slot, true, s, a0 + GROW_LOCAL, a1, lane))
       a1 = a0 + GROW_LOCAL;
@@ -754,12 +769,6 @@ union WarpScratch {
   MergeTile mg;
 };
 
-__device__ __forceinline__ uint32_t sel8(const uint4& a, const uint4& b, uint32_t i) {
-  const uint4& h = i < 4u ? a : b;
-  const uint32_t j = i & 3u;
-  return j == 0u ? h.x : (j == 1u ? h.y : (j == 2u ? h.z : h.w));
-}
-
 // Relax the arcs of the task's items [i0, i1), all of query q.  Lane j holds
 // in `x` the inclusive prefix n_0 + ... + n_j of the task's arc counts; item
 // i's arcs are [h[i].a0, h[i].a0 + n_i).  Every lane of the warp calls it with
@@ -802,17 +811,14 @@ __device__ __forceinline__ void relax_flat(const QDev& q, const RelaxHdr* __rest
       lim[u] = la.x;
       arc[u] = ok[u] ? __ldg(g.adj + la.y + (f - start)) : make_uint2(0u, 0u);
     }
-    uint4 ra[SSSP_U], rb[SSSP_U];
+    Row8 row[SSSP_U];
 #pragma unroll
     for (int u = 0; u < SSSP_U; u++) {
       ok[u] = ok[u] && arc[u].y <= lim[u];
-      if (ok[u]) {
-        const uint4* row = reinterpret_cast<const uint4*>(dist + (size_t)arc[u].x * 8);
-        ra[u] = __ldcg(row);
-        rb[u] = __ldcg(row + 1);
-      } else {
-        ra[u] = rb[u] = make_uint4(0u, 0u, 0u, 0u);
-      }
+      if (ok[u])
+        row[u] = ld_row(dist + (size_t)arc[u].x * ROW);
+      else
+        row[u] = Row8{};
     }
     uint32_t nn[SSSP_U], nf[SSSP_U];
 #pragma unroll
@@ -825,7 +831,7 @@ __device__ __forceinline__ void relax_flat(const QDev& q, const RelaxHdr* __rest
         const uint4 h0 = hv[0], h1 = hv[1];
         const uint32_t rm = h1.w;
         const uint32_t dv[KMAX] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z};
-        const uint32_t du[KMAX] = {ra[u].x, ra[u].y, ra[u].z, ra[u].w, rb[u].x, rb[u].y, rb[u].z};
+        const uint32_t(&du)[8] = row[u].w;
 #pragma unroll
         for (int t = 0; t < KMAX; t++) {
           if ((rm >> t) & 1u) {
@@ -860,7 +866,7 @@ __device__ __forceinline__ void relax_flat(const QDev& q, const RelaxHdr* __rest
       // the round: it filters repeated relaxations of a target far better
       // than the previous round's row, at the price of a few entries for
       // vertices whose own new value has not been carried across yet)
-      const uint32_t fw = rb[u].w;
+      const uint32_t fw = row[u].w[FLAGW];
       if (bits & ~fw) red_or(dist + (size_t)arc[u].x * ROW + FLAGW, bits);
       tN[u] = nn[u] && ((fw >> nsh) & 0xFFu) == 0u;
       tF[u] = nf[u] && ((fw >> FAR_SH) & 0xFFu) == 0u;
@@ -899,17 +905,11 @@ __device__ void sssp_task(const QDev* qd, const uint32_t* __restrict__ pre, int 
     const uint32_t psh = near_sh(q.par);
     const uint32_t m =
         (atomicAnd(q.dist + (size_t)v * ROW + FLAGW, ~(0xFFu << psh)) >> psh) & 0xFFu;
-    const uint4* drow = reinterpret_cast<const uint4*>(q.dist + (size_t)v * ROW);
-    const uint4 da = __ldcg(drow), db = __ldcg(drow + 1);
+    const Row8 dr = ld_row(q.dist + (size_t)v * ROW);
     uint32_t best = ld_best(q.ctl);
-    const uint32_t b0 = __ldg(g.beg + v), b1 = __ldg(g.beg + v + 1);
-    uint4 wa = make_uint4(b1, b1, b1, b1), wb = wa;
-    if (g.wcut != nullptr) {
-      const uint4* wr = reinterpret_cast<const uint4*>(g.wcut + (size_t)v * 8);
-      wa = __ldg(wr);
-      wb = __ldg(wr + 1);
-    }
-    const uint32_t d[KMAX] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z};
+    const Row8 cut = ld_row_nc(g.wcut + (size_t)v * 8);
+    const uint32_t b0 = cut.w[7];
+    const uint32_t(&d)[8] = dr.w;
     if (q.dist_nx != q.dist) {
       // exact rounds: the distances that changed last round carry over into
       // the rows this round writes (the other rows hold them already)
@@ -947,8 +947,7 @@ __device__ void sssp_task(const QDev* qd, const uint32_t* __restrict__ pre, int 
     uint32_t lim = 0;
     if (active) {
       lim = capb - dmin;
-      uint32_t a1 = b1;
-      if (g.wcut != nullptr && lim <= 128u) a1 = sel8(wa, wb, lim <= 1u ? 0u : 32u - __clz(lim - 1u));
+      const uint32_t a1 = arcs_end(g, v, cut, lim);
       n = a1 - b0;
       // hub: hand all but the first HUB_LOCAL arcs to k_heavy in chunks of
       // HUB_CHUNK arcs, one warp each
@@ -1018,10 +1017,9 @@ __device__ void hub_chunk(const QDev* qd, const uint4 item, const GraphDev& g, u
   const QDev& q = qd[slot];
   uint32_t capb = 0, n = 0;
   if (lane == 0) {
-    const uint4* drow = reinterpret_cast<const uint4*>(q.dist + (size_t)v * ROW);
-    const uint4 da = __ldcg(drow), db = __ldcg(drow + 1);
+    const Row8 dr = ld_row(q.dist + (size_t)v * ROW);
     const uint32_t best = ld_best(q.ctl);
-    const uint32_t d[KMAX] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z};
+    const uint32_t(&d)[8] = dr.w;
     capb = (uint32_t)((unsigned long long)best * q.cap_num / q.cap_den);
     uint32_t rm = 0, dmin = INF32;
 #pragma unroll
@@ -1075,8 +1073,10 @@ __device__ void grow_chunk(const QDev* qd, const uint4 item, const GraphDev& g, 
   lbv = __shfl_sync(FULL, lbv, 0);
   if (c == INF32 || c > best || !lb_ok(c, lbv, best)) return;
   if (!hop && 2ull * c > best) return;
+  const int64_t glim = grow_limit(q, comp, c, best);
+  if (glim <= 0) return;
   GrowCnt gc;
-  grow_arcs(q, g, lane, v, p, comp, c, best, best - c, hop ? (int)d + 1 : -1, item.z, item.w, gc, wb);
+  grow_arcs(q, g, lane, v, p, comp, c, best, (uint32_t)glim, hop ? (int)d + 1 : -1, item.z, item.w, gc, wb);
   const uint32_t a = warp_sum(gc.arcs), u = warp_sum(gc.upd), e = warp_sum(gc.enq);
   if (lane == 0) {
     ws_add(ws, q.ctl, ST_ARCS, a);
@@ -1114,9 +1114,9 @@ __device__ __forceinline__ uint32_t list_item(const QDev& q, uint32_t idx, uint3
 }
 
 __device__ __forceinline__ void load_row(const uint32_t* rows, uint32_t v, uint32_t (&r)[KMAX]) {
-  const uint4* p = reinterpret_cast<const uint4*>(rows + (size_t)v * ROW);
-  const uint4 a = __ldcg(p), b = __ldcg(p + 1);
-  r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w; r[4] = b.x; r[5] = b.y; r[6] = b.z;
+  const Row8 x = ld_row(rows + (size_t)v * ROW);
+#pragma unroll
+  for (int t = 0; t < KMAX; t++) r[t] = x.w[t];
 }
 
 // Lower m[] over up to PULL_U arcs a0 + i * stride (< a1) of weight <= lim;
@@ -1133,24 +1133,22 @@ __device__ __forceinline__ uint32_t pull_arcs(const GraphDev& g, const uint32_t*
     ok[u] = a < a1;
     arc[u] = ok[u] ? __ldg(g.adj + a) : make_uint2(0u, 0u);
   }
-  uint4 x[PULL_U], y[PULL_U];
+  Row8 x[PULL_U];
 #pragma unroll
   for (int u = 0; u < PULL_U; u++) {
-    x[u] = y[u] = make_uint4(INF32, INF32, INF32, INF32);
     if (ok[u] && arc[u].y <= lim) {
-      const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)arc[u].x * ROW);
-      x[u] = __ldcg(p);
-      y[u] = __ldcg(p + 1);
+      x[u] = ld_row(src + (size_t)arc[u].x * ROW);
       n++;
+    } else {
+      x[u] = Row8{{INF32, INF32, INF32, INF32, INF32, INF32, INF32, INF32}};
     }
   }
 #pragma unroll
   for (int u = 0; u < PULL_U; u++) {
-    const uint32_t r[KMAX] = {x[u].x, x[u].y, x[u].z, x[u].w, y[u].x, y[u].y, y[u].z};
 #pragma unroll
     for (int t = 0; t < KMAX; t++) {
-      const uint32_t d = r[t] + arc[u].y;
-      if (t < k && r[t] != INF32 && d <= capb) m[t] = min(m[t], d);
+      const uint32_t r = x[u].w[t], d = r + arc[u].y;
+      if (t < k && r != INF32 && d <= capb) m[t] = min(m[t], d);
     }
   }
   return n;
@@ -1185,8 +1183,8 @@ __device__ void pull_task(const QDev* qd, const uint32_t* __restrict__ pre, int 
     }
     if (!seen) {
       const uint32_t capb = ld_best(q.ctl);  // what exceeds the incumbent is as good as out of reach
-      const uint32_t a0 = __ldg(g.beg + v);
-      uint32_t a1 = arcs_upto(g, v, __ldg(g.beg + v + 1), capb);
+      uint32_t a0, a1;
+      arc_range(g, v, capb, a0, a1);
       const uint32_t n = a1 - a0;
       if (sd.big != nullptr && n >= sd.hub_min_deg && n - HUB_LOCAL >= sd.hub_min_rest) {
         const uint32_t st0 = a0 + HUB_LOCAL, nch = (a1 - st0 + HUB_CHUNK - 1u) / HUB_CHUNK;
@@ -1347,7 +1345,7 @@ __device__ void dseed_item(const QDev& q, uint32_t item) {
 // group b, then
 //   P[i][S][j]  cheapest visiting order of S starting at i, ending at j
 //   T2[i][S]    min_j P[i][S][j]
-// for the subsets S that hold i (replaces the host DP of DPQ.cu:409-483 /
+// for the subsets S that hold i, and the span table (replaces the host DP of DPQ.cu:409-483 /
 // AllPaths, CPUNONHOP.h:269-386).  Each warp works out gd again (a query has
 // few members; four of a lane's rows are in flight at once) and keeps it and
 // its 2^(k-1) x k table in shared memory: gd[64], Pi[2^(KMAX-1) * KMAX].  A
@@ -1410,11 +1408,22 @@ __device__ __noinline__ void tour_warp(const QDev& q, uint32_t i, uint32_t lane,
     const uint32_t c = t / k;
     P[subset(c) * k + (t - c * k)] = Pi[t];
   }
+  unsigned short* span = span_table(q);
   for (uint32_t c = lane; c < n; c += 32) {
-    uint32_t m = BIG;
-    for (uint32_t l = 0; l < k; l++) m = min(m, Pi[c * k + l]);
-    T2[subset(c)] = m;
+    const uint32_t S = subset(c);
+    uint32_t m = BIG, tour = BIG;
+    for (uint32_t l = 0; l < k; l++) {
+      m = min(m, Pi[c * k + l]);
+      tour = min(tour, sat_add(Pi[c * k + l], l == i ? 0u : min(gd[l * 8u + i], gd[i * 8u + l])));
+    }
+    T2[S] = m;
+    // half the cheapest closed tour of S (the same from each of its groups)
+    if ((S & ((1u << i) - 1u)) == 0u) {
+      const uint32_t half = (tour + 1u) >> 1;
+      span[S] = (unsigned short)(tour >= BIG ? LB_INF : min(half, LB_INF - 1u));
+    }
   }
+  if (i == 0u && lane == 0) span[0] = 0;
   __syncwarp();
 }
 
