@@ -149,7 +149,8 @@ struct alignas(64) QCtl {
   uint32_t n_far;    // append counter of the far list
   uint32_t n_far2;   // append counter of the far-out list (split rounds)
   uint32_t overflow; // a list exceeded its capacity
-  uint32_t pad1[4];
+  uint32_t deferred; // distance rounds: an item had arcs that lead beyond the reach
+  uint32_t pad1[3];
   // sectors 2-4: statistics
   unsigned long long stat[12];
   // sector 5: completion
@@ -189,6 +190,8 @@ struct QRun {
   uint32_t par;      // parity of the items in (or entering) the near list
   uint32_t lb_off;   // bound-table rows (vertices) already computed
   uint32_t win_items;  // items of the current window's rounds so far
+  uint32_t reach;      // unbounded distances: arcs that lead here or beyond are not relaxed yet
+  uint32_t rescan;     // this split round looks at every vertex (the reach has grown)
   // Hop-bounded distances: rounds 1..push_rounds relax from the vertices that
   // changed, the later ones gather at the few vertices that still need them
   // (see pull_task).  list h is qbuf[h]: the members (h = 0) and the vertices
@@ -251,6 +254,7 @@ struct GraphDev {
   // [V][8]: the first arc of v with weight > 2^b (b = 0..6), and in word 7 the
   // first arc of v: one row holds a vertex's whole range for most limits
   const uint32_t* wcut;
+  uint32_t wmax;         // heaviest arc
 };
 constexpr uint32_t WCUT_MAX = 64;  // largest limit the index bounds
 

@@ -70,6 +70,7 @@ static std::atomic<cudaError_t>& last_cuda_error() {
 struct gst_graph {
   uint32_t V = 0;
   uint64_t arcs = 0;
+  uint32_t wmax = 0;  // heaviest arc
   uint32_t* d_beg = nullptr;
   uint2* d_adj = nullptr;
   uint32_t* d_wcut = nullptr;  // per vertex: weight-bucket index (GraphDev::wcut)
@@ -1014,7 +1015,7 @@ class Runner {
   // static: the control step publishes the bound the round
   // kernels search, so the graph serves any set of admitted queries.
   gst_status build_round_graph() {
-    GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut};
+    GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut, g_->wmax};
     cudaGraph_t gr = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     cudaError_t le = cudaSuccess;
@@ -1055,7 +1056,7 @@ class Runner {
       tp.timeout_ns = (unsigned long long)(wm ? wm : wait_ms_default_) * 1000000ull;
       tp.hold = g_->hold_rounds.load();
       CK(cudaMemcpyAsync(d_pc_, &tp, sizeof(PersistCtl), cudaMemcpyHostToDevice, stream_));
-      GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut};
+      GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut, g_->wmax};
       // the control steps scan the slots in use: admissions happen only
       // between launches, so none above the highest one starts during it
       int nsc = (int)std::max<uint32_t>(1u, nslots_hi_);
@@ -1079,7 +1080,7 @@ class Runner {
       CK(cudaGraphLaunch(round_graph_, stream_));
     } else {
       // profiled blocks time every kernel with events between the launches
-      GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut};
+      GraphDev gd{g_->d_beg, g_->d_adj, g_->V, g_->d_wcut, g_->wmax};
       const int ns = (int)nslots_hi_;
       cudaEvent_t* pe = ev_prof_[h];
       for (uint32_t r = 0; r < R; r++) {
@@ -1353,6 +1354,11 @@ class ArcCheck {
   }
   ~ArcCheck() { join(); }
 
+  uint32_t heaviest() {
+    join();
+    return wmax_;
+  }
+
   bool ok() {
     join();
     if (!done_) {
@@ -1436,6 +1442,7 @@ gst_status build_adjacency(gst_graph* g, const uint32_t* beg, const uint32_t* cs
     CK(cudaStreamSynchronize(0));
   }
   if (!check.ok()) return GST_BAD_INPUT;
+  g->wmax = check.heaviest();
   unsigned long long* adj = reinterpret_cast<unsigned long long*>(g->d_adj);
   k_sort_lists<<<grid, 256>>>(g->d_beg, adj, V);
   CK(cudaGetLastError());
@@ -2245,7 +2252,7 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
     }
     if (n) CK(cudaMemcpy((uint32_t*)q.members + off, stage, n * 4, cudaMemcpyHostToDevice));
   }
-  GraphDev gd{g->d_beg, g->d_adj, g->V, g->d_wcut};
+  GraphDev gd{g->d_beg, g->d_adj, g->V, g->d_wcut, g->wmax};
   const uint32_t R = 2;  // most rounds are k_small's; what follows the last one is idle launches
   const uint64_t max_rounds = 1ull << 22;
   uint64_t rounds = 0;

@@ -936,17 +936,22 @@ __device__ void sssp_task(const QDev* qd, const uint32_t* __restrict__ pre, int 
     }
     // distances beyond cap(best) cannot lower a bound below best: skip them
     capb = (uint32_t)((unsigned long long)best * q.cap_num / q.cap_den);
-    uint32_t rm = 0, dmin = INF32;
+    // nor, for now, those from the reach on
+    const bool beyond = capb >= q.reach;
+    capb = min(capb, q.reach - 1u);
+    uint32_t rm = 0, dmin = INF32, dmax = 0;
 #pragma unroll
     for (int t = 0; t < KMAX; t++)
       if (t < k && ((m >> t) & 1u) && d[t] <= capb) {
         rm |= 1u << t;
         dmin = min(dmin, d[t]);
+        dmax = max(dmax, d[t]);
       }
     active = rm != 0;
     uint32_t lim = 0;
     if (active) {
       lim = capb - dmin;
+      if (beyond && capb - dmax < g.wmax && __ldca(&q.ctl->deferred) == 0u) q.ctl->deferred = 1u;
       const uint32_t a1 = arcs_end(g, v, cut, lim);
       n = a1 - b0;
       // hub: hand all but the first HUB_LOCAL arcs to k_heavy in chunks of
@@ -1020,7 +1025,7 @@ __device__ void hub_chunk(const QDev* qd, const uint4 item, const GraphDev& g, u
     const Row8 dr = ld_row(q.dist + (size_t)v * ROW);
     const uint32_t best = ld_best(q.ctl);
     const uint32_t(&d)[8] = dr.w;
-    capb = (uint32_t)((unsigned long long)best * q.cap_num / q.cap_den);
+    capb = min((uint32_t)((unsigned long long)best * q.cap_num / q.cap_den), q.reach - 1u);
     uint32_t rm = 0, dmin = INF32;
 #pragma unroll
     for (int t = 0; t < KMAX; t++)
@@ -1260,6 +1265,20 @@ __device__ void pull_chunk(const QDev* qd, const uint4 item, const GraphDev& g, 
 __device__ void split_item(const QDev& q, uint32_t s, bool& toN, bool& toF) {
   uint32_t best = ld_cg(&q.ctl->best);
   toN = toF = false;
+  if (q.phase == PH_SSSP && q.rescan) {
+    // item = a vertex: its distances are final, and arcs of theirs that led beyond
+    // the old reach are still to be relaxed, unless none stays under the cap
+    const uint32_t capb = (uint32_t)((unsigned long long)best * q.cap_num / q.cap_den);
+    uint32_t r[KMAX], nb = 0;
+    load_row(q.dist, s, r);
+#pragma unroll
+    for (int t = 0; t < KMAX; t++)
+      if (t < q.k && r[t] != INF32 && r[t] < capb) nb |= 1u << t;
+    // (the next round's parity, which a split round does not flip)
+    if (nb) red_or(q.dist + (size_t)s * ROW + FLAGW, nb << near_sh(q.par));
+    toN = nb != 0u;
+    return;
+  }
   if (q.phase == PH_SSSP) {
     uint32_t* fw = q.dist + (size_t)s * ROW + FLAGW;
     const uint32_t capb = (uint32_t)((unsigned long long)best * q.cap_num / q.cap_den);
@@ -1854,11 +1873,11 @@ __global__ void __launch_bounds__(256) k_init_workspace(const QDev* qd) {
 // What a control step reads of a query's control block, loaded at once: read
 // where they are needed, the words would cost a trip to L2 each.
 struct CtlIn {
-  uint32_t best, infeasible, center, n_near, n_far, n_far2, overflow, status, cancel;
+  uint32_t best, infeasible, center, n_near, n_far, n_far2, overflow, deferred, status, cancel;
   unsigned long long best_full;
   __device__ explicit CtlIn(const QCtl& c)
       : best(c.best), infeasible(c.infeasible), center(c.center), n_near(c.n_near), n_far(c.n_far), n_far2(c.n_far2),
-        overflow(c.overflow), status(c.status), cancel(c.cancel), best_full(c.best_full) {}
+        overflow(c.overflow), deferred(c.deferred), status(c.status), cancel(c.cancel), best_full(c.best_full) {}
 };
 
 // After a distance round of a hop-bounded query: the passes over its rows.
@@ -1981,7 +2000,14 @@ __device__ __forceinline__ void hop_rounds_done(QRun& q, QDev& qg, QCtl& c, cons
 // what is relaxed then (windows of 64 from the start cost six queries on 170k
 // vertices 5615 -> 6075 us); four times as wide after a window of at most
 // LIGHT_ITEMS items over all live queries, whose rounds are launch and latency;
-// and the rest in one window once an incumbent caps them.
+// and the rest in one window once an incumbent caps them.  Only arcs that lead
+// below the reach, two widths, are relaxed at first: without an incumbent a
+// vertex's heavy arcs lead to distances that almost never matter.  Should the
+// incumbent turn out beyond it (or none be found), every vertex reached relaxes
+// all its arcs once more.  The reach took 90 queries on 170k vertices from 15.5 to
+// 14.8 ms and 48 mixed ones on 3M from 104 to 96; relaxing below the window's own
+// end only, with a look at every vertex for each new window, halved the arcs but
+// cost the serving mixes 2-6%.
 constexpr uint32_t LIGHT_ITEMS = 16384;
 __device__ __forceinline__ uint32_t window_end(const QRun& q, uint32_t lo, uint32_t best, uint32_t limit) {
   uint32_t w = q.delta;
@@ -2003,6 +2029,7 @@ __device__ __forceinline__ void decide(QRun& q, QDev& qg, QCtl& c, const CtlIn& 
         // (one window holding everything): after D rounds every path of at
         // most D hops has been relaxed
         q.theta_hi = q.D >= 0 ? INF32 : q.delta_sssp;
+        q.reach = q.D >= 0 ? INF32 : (q.delta_sssp > BIG / 2u ? INF32 : 2u * q.delta_sssp);
         q.delta = q.delta_sssp;
         q.win_items = 0;
         q.hops = 0;
@@ -2052,13 +2079,22 @@ __device__ __forceinline__ void decide(QRun& q, QDev& qg, QCtl& c, const CtlIn& 
         // distance rounds only matter up to cap(best); DP rounds up to best
         unsigned long long limit = in.best;
         if (q.st == J_SSSP && in.best != INF32) limit = (unsigned long long)in.best * q.cap_num / q.cap_den;
-        bool exhausted = q.n_far == 0 || next_lo > limit;
+        // arcs beyond the reach are left: what comes next is every vertex again
+        const bool again = q.st == J_SSSP && q.n_far == 0 && in.deferred != 0u && limit >= q.reach;
+        bool exhausted = (q.n_far == 0 && !again) || next_lo > limit;
+        q.rescan = 0;
         if (!exhausted) {
+          if (again) {
+            q.rescan = 1;
+            q.reach = INF32;
+            c.deferred = 0;
+          }
           if (q.st == J_SSSP && (unsigned long long)q.win_items * n_live <= LIGHT_ITEMS && q.delta < BIG / 4u)
             q.delta *= 4u;
           q.win_items = 0;
           q.theta_lo = next_lo;
           q.theta_hi = window_end(q, next_lo, in.best, (uint32_t)limit);
+          if (q.st == J_SSSP) q.theta_hi = min(q.theta_hi, q.reach);
           c.n_near = 0;
           c.n_far2 = 0;
           q.act = A_SPLIT;
@@ -2067,7 +2103,8 @@ __device__ __forceinline__ void decide(QRun& q, QDev& qg, QCtl& c, const CtlIn& 
         if (q.st == J_SSSP) {
           if (q.D >= 0) hop_rounds_done(q, qg, c, in);  // its rounds converged before D
           // every distance below theta_hi is exact and every distance <=
-          // cap(best) was discovered; unknown ones are >= min(theta_hi, cap+1)
+          // cap(best), which is below the reach if arcs were left, was
+          // discovered; unknown ones are >= min(theta_hi, cap+1)
           unsigned long long b1 = in.best == INF32 ? (unsigned long long)INF32 : limit + 1;
           unsigned long long cap1 = q.n_far == 0 ? b1 : (q.theta_hi < b1 ? q.theta_hi : b1);
           q.cap1 = (uint32_t)(cap1 < BIG ? cap1 : BIG);
@@ -2170,7 +2207,7 @@ __device__ void control_step(QDev* qd, QCtl* ctl, int nslots, RoundDesc* rd, uin
         switch (q.act) {
           case A_SSEED:
           case A_DSEED: cnt[T_ITEM] = q.n_members; break;
-          case A_SPLIT: cnt[T_ITEM] = q.n_far; break;
+          case A_SPLIT: cnt[T_ITEM] = q.rescan ? q.nv : q.n_far; break;
           case A_PULL: {  // round hops + 1: the lists 0 .. D - (hops + 1)
             const uint32_t h = (uint32_t)q.D - q.hops - 1u;
             cnt[T_PULL] = h == 0u ? q.n_list[0] : (h == 1u ? n01 : (h == 2u ? n012 : n012 + q.n_list[3]));
@@ -2347,7 +2384,7 @@ __device__ __forceinline__ void light_task(const QDev* qd, const RoundDesc& sd, 
       const QDev& q = qd[slot];
       const uint32_t idx = it - __ldcg(P + slot);
       if (q.act == A_SPLIT) {
-        item = q.qbuf[q.far_idx][idx];
+        item = q.rescan ? idx : q.qbuf[q.far_idx][idx];
         split_item(q, item, toN, toF);
       } else if (q.act == A_SSEED) {
         const uint32_t m = __ldg(q.members + idx);

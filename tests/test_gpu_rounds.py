@@ -120,3 +120,60 @@ def test_staging_grows_for_large_member_lists(gst_lib, oracle_mod):
             else:
                 assert not O.validate(g, gr, q, -1, r.cost, r.root, r.edges)
     E.close()
+
+
+def _subset_dp(g, gr, q):
+    """Optimal cost by subset dynamic programming over all vertices, 64-bit (the
+    oracle's programs take costs from 100000 on for infinite); None: not connected."""
+    inf = 1 << 60
+    src = np.repeat(np.arange(g.V), np.diff(g.beg_pos.astype(np.int64)))
+    table = {}
+    for S in range(1, 1 << len(q)):
+        row = np.full(g.V, inf, dtype=np.int64)
+        if S & (S - 1) == 0:
+            row[gr.group(int(q[S.bit_length() - 1]))] = 0
+        A = (S - 1) & S
+        while A:
+            row = np.minimum(row, table[A] + table[S ^ A])
+            A = (A - 1) & S
+        while True:
+            new = np.minimum(row, inf)
+            np.minimum.at(new, g.csr, row[src] + g.weight)
+            if (new == row).all():
+                break
+            row = new
+        table[S] = row
+    best = int(table[(1 << len(q)) - 1].min())
+    return best if best < inf // 2 else None
+
+
+@pytest.mark.parametrize("wmax", (3, 40, 300, 1_000_000))
+def test_weights_beyond_the_reach(gst_lib, oracle_mod, wmax):
+    """Distances that end inside the first windows, beyond the reach of the first
+    rounds (two widths: every vertex then relaxes again), far beyond it, and
+    groups that are not connected at all (no incumbent ever ends the windows)."""
+    eng, O = gst_lib, oracle_mod
+    rng = np.random.default_rng(wmax)
+    V = 400
+    a, b = rng.integers(0, V - 20, size=(2, 1000))
+    keep = a != b
+    pairs = np.unique(np.stack([np.minimum(a, b), np.maximum(a, b)], 1)[keep], axis=0)
+    chain = np.stack([np.arange(V - 20, V - 1), np.arange(V - 19, V)], 1)  # a component of its own
+    pairs = np.concatenate([pairs, chain])
+    g = gen.csr_from_edges(V, pairs[:, 0], pairs[:, 1], rng.integers(1, wmax + 1, len(pairs)).astype(np.int32))
+    gr = gen.zipf_groups(V, 60, 1.5, 4, seed=wmax)
+    E = eng.Engine.from_instance(g, gr)
+    queries = [rng.choice(gr.n_groups, size=int(k), replace=False).astype(np.uint32)
+               for k in rng.integers(2, 6, size=24)]
+    res = E.query_batch(queries) + [E.query(q) for q in queries[:6]]
+    E.close()
+    bad = []
+    for q, r in zip(queries + queries[:6], res):
+        want = _subset_dp(g, gr, q)
+        if want is None:
+            bad += [] if r.status == eng.GST_NO_SOLUTION else [(q.tolist(), "want no solution", r.status, r.cost)]
+        elif r.status != eng.GST_OK or r.cost != want:
+            bad.append((q.tolist(), want, r.status, r.cost))
+        elif O.validate(g, gr, q, -1, r.cost, r.root, r.edges):
+            bad.append((q.tolist(), "invalid tree"))
+    assert not bad, bad[:10]
