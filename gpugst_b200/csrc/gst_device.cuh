@@ -353,41 +353,4 @@ __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) {
   return (s < a || s > BIG) ? BIG : s;
 }
 
-// Lower bound on the cost of connecting a vertex (with group distances dl[],
-// already capped) to every group of `comp`:
-//   one-label  max_j dl_j                                   (DPQ.cu:182-188)
-//   tour lb1   min_{i,j} ceil((dl_i + P[i][comp][j] + dl_j)/2)   (CPUNONHOP.h:448-466)
-//   tour lb2   max_i ceil((dl_i + T2[i][comp] + min_j dl_j)/2)   (CPUNONHOP.h:468-472)
-// P[i][S][j] = cheapest order of visiting the groups of S starting at i and
-// ending at j with group-to-group distances as step costs; T2 = min_j P.
-__device__ __forceinline__ uint32_t lower_bound_comp(const uint32_t (&dl)[KMAX], int k,
-                                                     uint32_t comp, const uint32_t* __restrict__ P,
-                                                     const uint32_t* __restrict__ T2) {
-  if (comp == 0) return 0;
-  const uint32_t K2 = 1u << k;
-  uint32_t lb0 = 0, mind = BIG;
-#pragma unroll
-  for (int j = 0; j < KMAX; j++)
-    if (j < k && (comp >> j & 1u)) {
-      lb0 = max(lb0, dl[j]);
-      mind = min(mind, dl[j]);
-    }
-  uint32_t lb1 = BIG, lb2 = 0;
-#pragma unroll
-  for (int i = 0; i < KMAX; i++) {
-    if (i < k && (comp >> i & 1u)) {
-      const uint32_t* Pi = P + ((size_t)i * K2 + comp) * k;
-#pragma unroll
-      for (int j = 0; j < KMAX; j++)
-        if (j < k && (comp >> j & 1u)) {
-          uint32_t t = sat_add(sat_add(dl[i], ld_round(Pi + j)), dl[j]);
-          lb1 = min(lb1, (t + 1) >> 1);
-        }
-      uint32_t t2 = sat_add(sat_add(dl[i], ld_round(T2 + (size_t)i * K2 + comp)), mind);
-      lb2 = max(lb2, (t2 + 1) >> 1);
-    }
-  }
-  return max(lb0, max(lb1 >= BIG ? BIG : lb1, lb2));
-}
-
 }  // namespace gstb

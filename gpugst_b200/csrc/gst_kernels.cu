@@ -756,10 +756,9 @@ struct RelaxCnt {
 };
 
 // Per-warp shared scratch; a warp uses one member at a time: the headers of
-// its distance items (or of a hub chunk), its bound rows' list and capped
-// distances, or a DP state's merge tile.
+// its distance items (or of a hub chunk), its bound rows' list, or a DP state's
+// merge tile.
 struct LbScratch {
-  uint32_t dl[KMAX][32];  // each lane's capped distances
   uint32_t v[64];         // live vertices still to evaluate, all of query `slot`
   uint32_t n, slot;
 };
@@ -1446,47 +1445,54 @@ __device__ __noinline__ void tour_warp(const QDev& q, uint32_t i, uint32_t lane,
   __syncwarp();
 }
 
-// lower_bound_comp for a subset X that every lane of the warp evaluates at
-// the same time: the loops run over the groups of X only, and lane `lane`'s
-// capped distances are read from shared memory (sdl[j][lane]), where a
-// group index that varies inside the loop costs no local memory.  Same value
-// as lower_bound_comp, with less work:
-//   - each unordered pair {i, j} is visited once with the cheaper of the two
-//     orders P[i][X][j], P[j][X][i] (the ordered pairs (i, j) and (j, i) give
-//     d_i + P[i][X][j] + d_j and d_j + P[j][X][i] + d_i); a pair (i, i) only
-//     exists for X = {i}, where every bound is d_i;
-//   - each term is a sum of three values <= 2^30, which cannot overflow 32
+// Lower bound on the cost of connecting a vertex (a lane's own, with group
+// distances d[], already capped) to every group of X:
+//   one-label  max_j d_j                                   (DPQ.cu:182-188)
+//   tour lb1   min_{i,j} ceil((d_i + P[i][X][j] + d_j)/2)   (CPUNONHOP.h:448-466)
+//   tour lb2   max_i ceil((d_i + T2[i][X] + min_j d_j)/2)   (CPUNONHOP.h:468-472)
+// P[i][S][j] = cheapest order of visiting the groups of S starting at i and
+// ending at j with group-to-group distances as step costs; T2 = min_j P.  Every
+// lane of the warp evaluates the same X, so the tests on it branch alike, the
+// table reads are one broadcast, and with the loops unrolled over all groups the
+// distances stay in registers.
+//   - Each unordered pair {i, j} is visited once, in the order i < j: a tour can be
+//     walked either way, so either order's P bounds it (they are equal unless one
+//     of two distances between the same groups was cut off above the cap).  A pair
+//     (i, i) only exists for X = {i}, where every bound is d_i.
+//   - Each term is a sum of three values <= 2^30, which cannot overflow 32
 //     bits, and saturation at BIG and the halving are monotone, so both are
 //     applied once to the minimum (lb1) or maximum (lb2) instead of per term.
-__device__ __forceinline__ uint32_t lower_bound_uniform(const uint32_t (*sdl)[32], uint32_t lane, int k, uint32_t X,
+// Against loops over the set bits with the distances in shared memory and both
+// orders read: 48 mixed queries on 3M vertices 96.9 -> 92.7 ms, two of k = 6, 7 on
+// 54k vertices 3144 -> 3027 us.
+__device__ __forceinline__ uint32_t lower_bound_uniform(const uint32_t (&d)[KMAX], int k, uint32_t X,
                                                         const uint32_t* __restrict__ P,
                                                         const uint32_t* __restrict__ T2) {
   const uint32_t K2 = 1u << k;
-  if ((X & (X - 1u)) == 0u) return sdl[__ffs(X) - 1][lane];  // a single group
   uint32_t lb0 = 0, mind = BIG;
-  for (uint32_t m = X; m; m &= m - 1u) {
-    const uint32_t d = sdl[__ffs(m) - 1][lane];
-    lb0 = max(lb0, d);
-    mind = min(mind, d);
-  }
-  uint32_t m1 = 0xFFFFFFFFu, m2 = 0;
-  for (uint32_t mi = X; mi; mi &= mi - 1u) {
-    const uint32_t i = __ffs(mi) - 1;
-    const uint32_t di = sdl[i][lane];
-    const uint32_t* Pi = P + ((size_t)i * K2 + X) * k;
-    for (uint32_t mj = mi & (mi - 1u); mj; mj &= mj - 1u) {  // the groups of X above i
-      const uint32_t j = __ffs(mj) - 1;
-      const uint32_t pij = min(ld_round(Pi + j), ld_round(P + ((size_t)j * K2 + X) * k + i));
-      m1 = min(m1, di + pij + sdl[j][lane]);
+#pragma unroll
+  for (int j = 0; j < KMAX; j++)
+    if (X >> j & 1u) {
+      lb0 = max(lb0, d[j]);
+      mind = min(mind, d[j]);
     }
-    m2 = max(m2, di + ld_round(T2 + (size_t)i * K2 + X) + mind);
-  }
+  if ((X & (X - 1u)) == 0u) return lb0;  // a single group
+  uint32_t m1 = 0xFFFFFFFFu, m2 = 0;
+#pragma unroll
+  for (int i = 0; i < KMAX; i++)
+    if (X >> i & 1u) {
+      const uint32_t* Pi = P + ((size_t)i * K2 + X) * k;
+#pragma unroll
+      for (int j = i + 1; j < KMAX; j++)
+        if (X >> j & 1u) m1 = min(m1, d[i] + ld_round(Pi + j) + d[j]);
+      m2 = max(m2, d[i] + ld_round(T2 + (size_t)i * K2 + X) + mind);
+    }
   const uint32_t lb1 = (min(m1, BIG) + 1u) >> 1;
   const uint32_t lb2 = (min(m2, BIG) + 1u) >> 1;
   return max(lb0, max(lb1, lb2));
 }
 
-// Lower-bound table rows: lbt[v][X] = lower_bound_comp(d(v), X) for every
+// Lower-bound table rows: lbt[v][X] = lower_bound_uniform(d(v), X) for every
 // subset X (the per-vertex one_label_lb table of the reference,
 // DPQ.cu:174-224, with the tour bounds of CPUNONHOP.h:436-496), saturated to
 // 16 bits, which only lowers a bound.  A warp first looks 32 consecutive
@@ -1509,8 +1515,8 @@ __device__ __forceinline__ uint32_t lower_bound_uniform(const uint32_t (*sdl)[32
 // at admission: six hop-bounded queries on 2^20 vertices 5.5 -> 4.1 ms (their
 // starts had differed by launches alone before), 48 of them in a batch 34.9 ->
 // 27.2 ms, 48 mixed queries on 3M vertices 226 -> 202 ms.
-__device__ __forceinline__ void lb_stage_row(const QDev& q, bool mine, uint32_t v, uint32_t lane,
-                                             uint32_t (*sdl)[32], uint32_t& dmin, uint32_t& dmax) {
+__device__ __forceinline__ void lb_row(const QDev& q, bool mine, uint32_t v,
+                                             uint32_t (&d)[KMAX], uint32_t& dmin, uint32_t& dmax) {
   uint32_t r[KMAX] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
   if (mine) {
     load_row(q.dist, v, r);
@@ -1546,11 +1552,10 @@ __device__ __forceinline__ void lb_stage_row(const QDev& q, bool mine, uint32_t 
   dmax = 0u;
 #pragma unroll
   for (int j = 0; j < KMAX; j++) {
-    const uint32_t d = min(r[j], q.cap1);
-    sdl[j][lane] = d;
+    d[j] = min(r[j], q.cap1);
     if (j < q.k) {
-      dmin = min(dmin, d);
-      dmax = max(dmax, d);
+      dmin = min(dmin, d[j]);
+      dmax = max(dmax, d[j]);
     }
   }
 }
@@ -1564,30 +1569,26 @@ __device__ void lb_eval(const QDev* qd, uint32_t cnt, uint32_t lane, LbScratch& 
   const uint32_t* T2 = q.tour + (size_t)k * K2 * k;
   const bool mine = lane < cnt;
   const uint32_t v = mine ? lb.v[lane] : 0u;
-  uint32_t dmin, dmax;
-  lb_stage_row(q, mine, v, lane, lb.dl, dmin, dmax);
-  __syncwarp();
+  uint32_t d[KMAX], dmin, dmax;
+  lb_row(q, mine, v, d, dmin, dmax);
   unsigned short* out = q.lbt + ((size_t)v << k);
   for (uint32_t x0 = 0; x0 < K2; x0 += 8u) {
-    uint32_t pk[4];
+    unsigned long long pk[2] = {0, 0};  // eight entries
 #pragma unroll
-    for (int h = 0; h < 4; h++) {
-      uint32_t two = 0;
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const uint32_t X = x0 + 2u * h + e;
+    for (int h = 0; h < 2; h++)
+#pragma unroll 1
+      for (uint32_t e = 0; e < 4u; e++) {
+        const uint32_t X = x0 + 4u * h + e;
         uint32_t bound = 0;
-        if (X != 0u && X < K2) bound = lower_bound_uniform(lb.dl, lane, k, X, P, T2);
+        if (X != 0u && X < K2) bound = lower_bound_uniform(d, k, X, P, T2);
         const uint32_t ent = bound >= BIG ? LB_INF : min(bound, LB_INF - 1u);
-        two |= ent << (16 * e);
+        pk[h] |= (unsigned long long)ent << (16u * e);
       }
-      pk[h] = two;
-    }
     if (mine) {
       if (K2 >= 8u) {
-        *reinterpret_cast<uint4*>(out + x0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        *reinterpret_cast<ulonglong2*>(out + x0) = make_ulonglong2(pk[0], pk[1]);
       } else {
-        for (uint32_t X = 0; X < K2; X++) out[X] = (unsigned short)(pk[X >> 1] >> (16 * (X & 1u)));
+        for (uint32_t X = 0; X < K2; X++) out[X] = (unsigned short)(pk[0] >> (16u * X));
       }
     }
   }
@@ -1623,13 +1624,12 @@ __device__ void lbt_rows32(const QDev* qd, const uint32_t* __restrict__ pre, int
     const uint32_t K2 = 1u << k;
     if (lb.n != 0u && lb.slot != si) lb_flush(qd, lane, lb);
     const uint32_t v = mine ? q.lb_off + (it - pre[si]) : 0u;
-    uint32_t dmin, dmax;
-    lb_stage_row(q, mine, v, lane, lb.dl, dmin, dmax);
-    __syncwarp();
+    uint32_t d[KMAX], dmin, dmax;
+    lb_row(q, mine, v, d, dmin, dmax);
     const uint32_t best = ld_best(q.ctl);
     bool live = mine && dmax < BIG && (dmin == 0u || dmin + dmax <= best);
     if (__any_sync(FULL, live)) {
-      const uint32_t all = lower_bound_uniform(lb.dl, lane, k, K2 - 1u, q.tour, q.tour + (size_t)k * K2 * k);
+      const uint32_t all = lower_bound_uniform(d, k, K2 - 1u, q.tour, q.tour + (size_t)k * K2 * k);
       live = live && all < BIG && all <= best;
     }
     const unsigned mm = __ballot_sync(FULL, mine), am = __ballot_sync(FULL, live);
