@@ -170,8 +170,10 @@ gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, int k, int D,
  * of them changes a result, only the work schedule and how tight the lower
  * bounds are. */
 typedef struct gst_tuning {
-  uint32_t delta_sssp;   /* width of the distance rounds' near-far window */
-  uint32_t delta_dp;     /* width of the DP rounds' near-far window */
+  uint32_t delta_sssp;   /* width of the distance rounds' first near-far window (later ones follow
+                            the incumbent; arcs that lead two widths off wait until it asks for them) */
+  uint32_t delta_dp;     /* width of the DP rounds' near-far windows in progressive mode (an exact
+                            query's first window reaches up to the incumbent, or 16 widths without one) */
   uint32_t hub_min_deg;  /* a vertex with this many arcs to relax hands them out in chunks (>= 32) */
   uint32_t cap_pct;      /* distances are computed exactly up to this percentage of the incumbent (1..100) */
   uint32_t persistent;   /* 1: each block of rounds is one persistent cooperative launch (the round
@@ -285,8 +287,9 @@ const char* gst_last_cuda_error(void);
  * graph's engine so far, and, when profiling is on (gst_query_batch calls
  * only), the accumulated device time of the round kernels
  * (kernel_ms[0] = k_light: distance items, splits, seeds, tours,
- * extraction, DP states; kernel_ms[1] = k_heavy: arc chunks, lower-bound
- * rows, snapshots; when the rounds ran as persistent launches,
+ * extraction, DP states, gathered rows; kernel_ms[1] = k_heavy: arc chunks,
+ * lower-bound rows, passes over distance rows; while profiling, no round runs
+ * inside the control kernel; when the rounds ran as persistent launches,
  * kernel_ms[0] = k_rounds, all of the round, and kernel_ms[1] = 0), the
  * number of rounds, and the summed GST_STAT_* counters of finished queries. */
 uint64_t gst_kernel_launches(const gst_graph* g);
