@@ -1814,9 +1814,10 @@ __device__ __noinline__ void extract_warp(const QDev& q, const GraphDev& g, uint
 // them: blockIdx.y is the query, whose record in `stage` (at off[y]) is its
 // descriptor, its control block and its member items, each 64-byte aligned.
 // Descriptor and control block go to the query's slot and the members to its
-// workspace; both distance-row buffers are set to "unknown" (words 0..6 all
-// ones) with no group pending (word 7 zero), and, for k < 3, the state flags to
-// zero (a vertex's flags are not whole words then).  The state table, up to
+// workspace; the distance rows that the rounds will read are set to "unknown"
+// (words 0..6 all ones) with no group pending (word 7 zero), and, for k < 3, the
+// state flags to zero (a vertex's flags are not whole words then).  The state
+// table, up to
 // 7.7 GB at 3M vertices, is not touched: the bound-row pass fills the rows of the
 // vertices that can hold a state.  Bound by its HBM writes for large graphs (64
 // bytes a vertex) and by its launch for small ones.  A kernel and three copies
@@ -1825,16 +1826,29 @@ __device__ __noinline__ void extract_warp(const QDev& q, const GraphDev& g, uint
 // 90-query batch on 170k vertices 19.8 -> 17.4 ms, 48 hop-bounded queries on
 // 2^20 vertices 4.07 -> 3.18 ms, one query on 10k vertices 493 -> 410 us.
 // ---------------------------------------------------------------------------
-__device__ void init_rows(const QDev& q, size_t tid, size_t stride) {
+__device__ void init_rows(const QDev& q, const uint32_t* members, size_t tid, size_t stride) {
   const uint4 ones = make_uint4(INF32, INF32, INF32, INF32);
   const uint4 tail = make_uint4(INF32, INF32, INF32, 0u);
   uint4* dist = reinterpret_cast<uint4*>(q.dist);
-  uint4* dist2 = q.dist_nx != q.dist ? reinterpret_cast<uint4*>(q.dist_nx) : nullptr;
+  uint4* next = reinterpret_cast<uint4*>(q.dist_nx);
+  // Unbounded queries have one buffer.  Of a hop-bounded query's two, the first is
+  // read and written at the members only when there is one relaxed round
+  // (D = 1..3), and the second not at all when there is none (D = 0).  Measured
+  // against both buffers always: one query (D = 2..4) on 2^20 vertices 1457 ->
+  // 1417 us, 48 in a batch 3.01 -> 2.86 ms; on 10k vertices the same.
+  const bool first = q.push_rounds != 1u || members == nullptr;
+  const bool second = next != dist && q.push_rounds != 0u;
   for (size_t i = tid; i < 2 * (size_t)q.nv; i += stride) {
     const uint4 x = (i & 1u) ? tail : ones;
-    dist[i] = x;
-    if (dist2 != nullptr) dist2[i] = x;
+    if (first) dist[i] = x;
+    if (second) next[i] = x;
   }
+  if (!first)
+    for (size_t i = tid; i < q.n_members; i += stride) {
+      uint4* row = dist + 2 * (size_t)(members[i] >> 3);
+      row[0] = ones;
+      row[1] = tail;
+    }
   if (q.k < 3)
     for (size_t i = tid; i < ((size_t)q.nv * q.WT + 7) / 8; i += stride) q.dflag[i] = 0u;
 }
@@ -1856,13 +1870,14 @@ __global__ void __launch_bounds__(256) k_admit(const unsigned char* __restrict__
   }
   uint32_t* members = const_cast<uint32_t*>(q.members);
   for (size_t i = tid; i < q.n_members; i += stride) members[i] = rm[i];
-  init_rows(q, tid, stride);
+  init_rows(q, rm, tid, stride);
 }
 
-// The same for the allocation-free query, whose descriptor, control block and
-// members are in place already.
+// The same for the allocation-free query, whose descriptor and control block are
+// in place already.  Its members may still be on their way (the copy overlaps
+// this: waiting for it cost 2 us of 548), so all of the first buffer is set.
 __global__ void __launch_bounds__(256) k_init_workspace(const QDev* qd) {
-  init_rows(*qd, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
+  init_rows(*qd, nullptr, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
