@@ -1819,8 +1819,8 @@ __device__ __noinline__ void extract_warp(const QDev& q, const GraphDev& g, uint
 // state flags to zero (a vertex's flags are not whole words then).  The state
 // table, up to
 // 7.7 GB at 3M vertices, is not touched: the bound-row pass fills the rows of the
-// vertices that can hold a state.  Bound by its HBM writes for large graphs (64
-// bytes a vertex) and by its launch for small ones.  A kernel and three copies
+// vertices that can hold a state.  Bound by its HBM writes for large graphs (32
+// bytes a vertex and buffer) and by its launch for small ones.  A kernel and three copies
 // for each query, two more copies for each finished one and a wait for the block
 // launched ahead, against this and trees written to the host by extraction: a
 // 90-query batch on 170k vertices 19.8 -> 17.4 ms, 48 hop-bounded queries on
