@@ -360,7 +360,9 @@ __device__ __forceinline__ void grow_arcs(const QDev& q, const GraphDev& g, uint
 // A warp hands the arcs [a0, a1) of a state's grow to k_heavy in HUB_CHUNK
 // pieces.  Entries below the list's capacity are always written (empty
 // ranges when the run does not fit), so k_heavy never reads a stale entry.
-// Returns false if the run did not fit: the caller then grows those arcs.
+// Returns false if the run did not fit: the caller then grows those arcs.  The
+// caller keeps the first GROW_LOCAL arcs, so it needs more than that, also where
+// the threshold (hub_min_deg, 32 or more) is lower.
 constexpr uint32_t CH_GROW = 1u << 31;  // big-list entry is a DP grow chunk
 constexpr uint32_t CH_HOP = 1u << 30;   // ... of a hop-bounded state
 
@@ -504,7 +506,7 @@ __device__ void dp_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_t
     const uint32_t lim = (uint32_t)glim;
     uint32_t a0, a1;
     arc_range(g, v, lim, a0, a1);
-    if (sd.grow_chunks && a1 - a0 >= sd.hub_min_deg &&
+    if (sd.grow_chunks && a1 - a0 >= max(sd.hub_min_deg, GROW_LOCAL + 1u) &&
         push_grow_chunks(sd, rd, slot, false, s, a0 + GROW_LOCAL, a1, lane))
       a1 = a0 + GROW_LOCAL;
     grow_arcs(q, g, lane, v, p, comp, c, best, lim, -1, a0, a1, gc, wb);
@@ -616,7 +618,7 @@ __device__ void hop_expand(const QDev& q, const GraphDev& g, uint32_t s, uint32_
     const uint32_t lim = (uint32_t)glim;
     uint32_t a0, a1;
     arc_range(g, v, lim, a0, a1);
-    if (sd.grow_chunks && a1 - a0 >= sd.hub_min_deg &&
+    if (sd.grow_chunks && a1 - a0 >= max(sd.hub_min_deg, GROW_LOCAL + 1u) &&
         push_grow_chunks(sd, rd, slot, true, s, a0 + GROW_LOCAL, a1, lane))
       a1 = a0 + GROW_LOCAL;
     grow_arcs(q, g, lane, v, p, comp, c, best, lim, (int)d + 1, a0, a1, gc, wb);

@@ -174,7 +174,8 @@ typedef struct gst_tuning {
                             the incumbent; arcs that lead two widths off wait until it asks for them) */
   uint32_t delta_dp;     /* width of the DP rounds' near-far windows in progressive mode (an exact
                             query's first window reaches up to the incumbent, or 16 widths without one) */
-  uint32_t hub_min_deg;  /* a vertex with this many arcs to relax hands them out in chunks (>= 32) */
+  uint32_t hub_min_deg;  /* a vertex with this many arcs to relax hands them out in chunks (>= 32; the
+                            grow of a DP state at it only beyond 128 arcs) */
   uint32_t cap_pct;      /* distances are computed exactly up to this percentage of the incumbent (1..100) */
   uint32_t persistent;   /* 1: each block of rounds is one persistent cooperative launch (the round
                             loop runs on the device, every block resident); 0: a CUDA graph of
