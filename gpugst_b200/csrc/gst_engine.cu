@@ -198,7 +198,7 @@ struct Job {
   uint32_t retries = 0;      // runs repeated after GST_QUEUE_OVERFLOW
   gst_status status = GST_OK;
   bool rejected = false;  // failed validation before admission
-  bool cancelled = false; // withdrawn while waiting for a rerun
+  bool cancelled = false; // withdrawn: not to be rerun
   bool done = false;
   bool early_done = false;   // fill_result has settled the progressive answer
   uint32_t lower_bound = 0;  // proven lower bound on the optimum
@@ -845,10 +845,22 @@ class Runner {
     return true;
   }
 
-  // Send the queries admitted since the last call to the device: one copy of
-  // their records (and of the list of their offsets) and one launch.
+  // Send the queries admitted since the last call to the device, then the cancel
+  // flags of the withdrawn ones.
   gst_status flush_admissions() {
-    if (staged_.empty()) return GST_OK;
+    if (!staged_.empty()) {
+      const gst_status st = flush_staged();
+      if (st != GST_OK) return st;
+    }
+    for (uint32_t s : cancel_slots_)
+      CK(cudaMemcpyAsync(&d_ctl_[s].cancel, h_one_, sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+    cancel_slots_.clear();
+    return GST_OK;
+  }
+
+  // One copy of the staged records (and of the list of their offsets) and one
+  // launch.
+  gst_status flush_staged() {
     const int sh = (int)(next_block_ & 1);
     char* half = h_stage_ + (size_t)sh * (stage_cap_ / 2);
     const size_t first = staged_.front(), list = stage_off_[sh], bytes = staged_.size() * 4;
@@ -870,25 +882,23 @@ class Runner {
     j->mem = nullptr;
   }
 
-  // Withdraw the admitted job with this tag: its control block's cancel flag
-  // is set stream-ordered after the block in flight, and the control step ends the
-  // job at its next round with GST_CANCELLED.  False if no admitted job has
-  // the tag (the caller checks its pending queue).
+  // Withdraw the admitted job with this tag.  On the device, flush_admissions
+  // sets its control block's cancel flag (after the admissions that it sends, as
+  // the job may be one of them: a rerun staged in the same iteration), and the
+  // control step ends the job at its next round with GST_CANCELLED.  A job whose
+  // run has ended, seen by the host or not, keeps its result, but is reported as
+  // cancelled instead of being rerun.  False if no admitted job has the tag (the
+  // caller checks its pending queue).
   bool cancel_tag(uint64_t tag) {
     for (Job* j : retry_)
-      if (j->tag == tag) {
-        j->cancelled = true;  // reported as cancelled instead of being rerun
-        return true;
-      }
+      if (j->tag == tag) return j->cancelled = true;
+    for (Job* j : fin_)
+      if (j->tag == tag) return j->cancelled = true;
     for (uint32_t s = 0; s < slots_.size(); s++) {
       Job* j = slots_[s];
       if (j && j->tag == tag) {
-        if (cudaMemcpyAsync(&d_ctl_[s].cancel, h_one_, sizeof(uint32_t), cudaMemcpyHostToDevice, stream_) !=
-            cudaSuccess) {
-          last_cuda_error() = cudaGetLastError();
-          return false;
-        }
-        return true;
+        cancel_slots_.push_back(s);
+        return j->cancelled = true;
       }
     }
     return false;
@@ -909,8 +919,9 @@ class Runner {
   gst_status run(AdmitFn&& admit_more, DoneFn&& on_done) {
     CK(cudaEventRecord(ev_[0], stream_));
     int64_t inflight = -1;  // id of the block launched but not yet examined
-    std::vector<Job*> fin;  // retired jobs whose tree copies are in flight
+    std::vector<Job*>& fin = fin_;
     std::vector<size_t> fin_off;
+    fin.clear();
     int fin_half = 0, seen_half = -1;
     using clk = std::chrono::steady_clock;
     auto ms_since = [](clk::time_point a) { return std::chrono::duration<double, std::milli>(clk::now() - a).count(); };
@@ -1233,6 +1244,7 @@ class Runner {
   gst_tuning tune_{};  // the launch parameters this runner admits queries with
   Arena arena_;
   std::deque<Job*> retry_;  // queries to run again with larger frontier lists
+  std::vector<Job*> fin_;   // retired jobs whose tree copies are in flight
   cudaStream_t stream_ = nullptr;
   std::vector<Job*> slots_;
   uint32_t n_used_ = 0, nslots_hi_ = 0, max_slots_ = MAX_SLOTS - 1;
@@ -1252,6 +1264,7 @@ class Runner {
   char* h_stage_ = nullptr;
   unsigned char* d_stage_ = nullptr;
   std::vector<uint32_t> staged_;  // offsets of the records staged and not yet sent
+  std::vector<uint32_t> cancel_slots_;  // slots whose cancel flag is not yet sent
   uint32_t* h_small_edges_ = nullptr;  // [slot][HOST_EDGES][3], written by extraction
   char* h_edge_stage_ = nullptr;
   size_t stage_cap_ = 0, stage_max_ = 0, stage_off_[2] = {0, 0}, edge_stage_cap_ = 0;
