@@ -187,6 +187,7 @@ struct Job {
   int nd = 1;
   uint32_t WT = 0, full = 0;
   size_t table_bytes = 0, bytes = 0;
+  size_t charged = 0;  // bytes counted against a server's budget so far (a rerun's workspace is larger)
   std::vector<uint32_t> members;
   // device workspace
   char* mem = nullptr;
@@ -902,6 +903,15 @@ class Runner {
       }
     }
     return false;
+  }
+
+  // Every job between its admission and its on_done call.
+  template <class F>
+  void for_each_admitted(F&& f) {
+    for (uint32_t s = 0; s < nslots_hi_; s++)
+      if (slots_[s]) f(slots_[s]);
+    for (Job* j : fin_) f(j);
+    for (Job* j : retry_) f(j);
   }
 
   double last_call_ms() const { return last_call_ms_; }
@@ -1891,6 +1901,10 @@ static void serve_loop(gst_server* S) {
           std::lock_guard<std::mutex> lk(S->mu);
           for (uint64_t id : S->cancels) S->runner->cancel_tag(id);
           S->cancels.clear();
+          S->runner->for_each_admitted([&](Job* j) {
+            S->in_use += j->bytes - j->charged;
+            j->charged = j->bytes;
+          });
           while (!S->pending.empty() && S->inflight < S->max_inflight && S->runner->has_free_slot()) {
             Job* j = S->pending.front();
             if (S->in_use + j->bytes > S->budget && S->inflight > 0) break;  // wait for memory
@@ -1909,14 +1923,14 @@ static void serve_loop(gst_server* S) {
             }
             S->pending.pop_front();
             S->inflight++;
-            S->in_use += j->bytes;
+            S->in_use += j->charged = j->bytes;
             S->running.insert(j->tag);
           }
         },
         [&](Job* j) {
           std::lock_guard<std::mutex> lk(S->mu);
           S->inflight--;
-          S->in_use -= j->bytes;
+          S->in_use -= j->charged;
           {
             auto it = S->running.find(j->tag);
             if (it != S->running.end()) S->running.erase(it);

@@ -68,3 +68,22 @@ def test_cancel_of_a_request_that_is_rerun(gst_lib, monkeypatch):
     assert not lost, (len(lost), lost[:10])
     assert st["cancelled"] == n and st["completed"] == n and st["inflight"] == 0
     assert last.status == eng.GST_OK and last.stats["retries"] > 0 and last.cost == 100 * (g.V - 1)
+
+
+def test_bytes_in_use_of_rerun_requests(gst_lib, monkeypatch):
+    """A rerun's workspace is larger than the one the request was admitted with;
+    once all is done, nothing is in use."""
+    eng = gst_lib
+    g, gr = _rerun_instance()
+    monkeypatch.setenv("GSTB_QUEUE_CAP", "1")
+    E = eng.Engine.from_instance(g, gr)
+    S = eng.Server(E, max_inflight=4)
+    q = np.array([0, 1, 2], dtype=np.uint32)
+    for i in range(8):
+        assert S.submit(i, q) == eng.GST_OK
+    got = _poll_all(S, 8)
+    st = S.stats()
+    S.close()
+    E.close()
+    assert all(r.status == eng.GST_OK and r.stats["retries"] > 0 for r in got.values()) and len(got) == 8
+    assert st["inflight"] == 0 and st["in_use_bytes"] == 0
