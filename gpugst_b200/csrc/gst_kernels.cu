@@ -1868,7 +1868,9 @@ __global__ void __launch_bounds__(256) k_admit(const unsigned char* __restrict__
       reinterpret_cast<unsigned long long*>(qd + slot)[i] = reinterpret_cast<const unsigned long long*>(rec)[i];
     for (uint32_t i = threadIdx.x; i < sizeof(QCtl) / 8; i += blockDim.x)
       reinterpret_cast<unsigned long long*>(q.ctl)[i] = reinterpret_cast<const unsigned long long*>(rc)[i];
-    if (threadIdx.x == 0) rd->n_live = 1u;  // the next control step has something to look at
+    // one more for the next control step to look at, beside those that the last
+    // one left running (the distance windows go by the number of live queries)
+    if (threadIdx.x == 0) atomicAdd(&rd->n_live, 1u);
   }
   uint32_t* members = const_cast<uint32_t*>(q.members);
   for (size_t i = tid; i < q.n_members; i += stride) members[i] = rm[i];

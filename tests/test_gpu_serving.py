@@ -87,3 +87,36 @@ def test_bytes_in_use_of_rerun_requests(gst_lib, monkeypatch):
     E.close()
     assert all(r.status == eng.GST_OK and r.stats["retries"] > 0 for r in got.values()) and len(got) == 8
     assert st["inflight"] == 0 and st["in_use_bytes"] == 0
+
+
+def test_windows_count_every_live_query(gst_lib):
+    """The distance windows widen after a window with few items over all live
+    queries.  Two queries whose every window is too large for that, with a third
+    kept busy by small ones that come and go, run exactly the rounds that they run
+    without them.
+
+    The graph is 40 layers of 12000 vertices, 16 apart, and each window (16 wide
+    at the start) holds one layer: 12000 items are few, 24000 are not.  The large
+    queries have no solution, so nothing but the windows paces them."""
+    eng = gst_lib
+    n, layers = 12000, 40
+    V = n * layers + 1
+    a = np.arange(n * (layers - 1))
+    nxt = (a // n + 1) * n
+    u = np.concatenate([a, a])
+    v = np.concatenate([nxt + a % n, nxt + (a + 1) % n])
+    g = gen.csr_from_edges(V, u, v, np.full(len(u), 16, dtype=np.int32))
+    gr = gen.Groups(np.array([0, n, n + 1, n + 2], dtype=np.uint64),
+                    np.concatenate([np.arange(n), [V - 1, V // 2]]).astype(np.uint32))
+    E = eng.Engine.from_instance(g, gr)
+    E.set_tuning(rounds_per_launch=1)
+    large, small = np.array([0, 1], dtype=np.uint32), np.array([2], dtype=np.uint32)
+    alone = E.query_batch([large, large])
+    # small ones of 5 to 7 rounds, so that their admissions meet the windows' ends too
+    mixed = E.query_batch([large, large] + [small] * 40, [-1, -1] + [-1, 0, 1, 2] * 10, max_concurrent=3)
+    E.close()
+    assert [r.status for r in alone + mixed[:2]] == [eng.GST_NO_SOLUTION] * 4
+    assert all(r.status == eng.GST_OK and r.cost == 0 for r in mixed[2:])
+    rounds = [r.stats["rounds"] for r in alone + mixed[:2]]
+    assert rounds[0] == rounds[1] > 2 * layers - 10, rounds
+    assert rounds[2:] == rounds[:2], rounds
