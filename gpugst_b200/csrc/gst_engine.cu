@@ -428,11 +428,22 @@ class Arena {
   std::atomic<int>* fail_ = nullptr;
 };
 
+// Entries that no frontier list of a query can exceed.  DP states are listed
+// once (their flags are taken with the old word returned), vertices in the
+// distance rounds not quite: threads that lower a vertex before any of them sees
+// its pending flag each list it, at most once for each arc relaxed, so a round
+// lists at most every vertex and every arc.
+uint64_t list_bound(const gst_graph* g, uint32_t WT) {
+  return std::min<uint64_t>(std::max<uint64_t>((uint64_t)g->V * WT, g->V + g->arcs), 1ull << 31);  // 32-bit indices
+}
+
 // Workspace layout of one query (see gst_device.cuh).
 struct Layout {
   size_t table, dist, dist2, dflag, qbuf, tour, lbt, extra, members, edges, total;
   uint32_t cap;
 };
+
+uint64_t list_cap_limit() { return env_u32("GSTB_QUEUE_CAP", 1u << 25); }
 
 // cap_req > 0 asks for a frontier-list capacity of that many items (a query
 // retried after GST_QUEUE_OVERFLOW); 0 takes the default.
@@ -441,10 +452,10 @@ Layout layout_for(const gst_graph* g, int k, int D, size_t n_members, uint32_t m
   Layout L{};
   uint64_t WT = (uint64_t)(1u << k) * nd;
   uint64_t states = (uint64_t)g->V * WT;
-  uint64_t caplim = env_u32("GSTB_QUEUE_CAP", 1u << 25);
-  // distance lists hold each vertex at most once per list (cap >= V never
-  // overflows there); DP lists start at a quarter of the states and grow by
-  // rerunning the query if a frontier outgrows them
+  uint64_t caplim = list_cap_limit();
+  // lists start at a quarter of the states and grow by rerunning the query if a
+  // frontier outgrows them (DP states of a dense query; vertices listed several
+  // times in a dense graph, see list_bound)
   uint64_t cap = std::min<uint64_t>(std::max<uint64_t>(states / 4, (uint64_t)g->V + 1024), caplim);
   if (cap_req) cap = cap_req;
   cap = std::max<uint64_t>(cap, 1024);
@@ -1227,8 +1238,7 @@ class Runner {
     auto now = std::chrono::steady_clock::now();
     for (size_t i = 0; i < fin.size(); i++) {
       Job* j = fin[i];
-      // lists of one entry per state cannot overflow; list indices are 32-bit
-      const uint64_t cap_max = std::min<uint64_t>((uint64_t)g_->V * j->WT, 1ull << 31);
+      const uint64_t cap_max = list_bound(g_, j->WT);
       if (j->status == GST_QUEUE_OVERFLOW && (uint64_t)j->qd.cap < cap_max) {
         // a frontier outgrew its list: run the query again with 4x the capacity
         j->cap_req = std::min<uint64_t>(cap_max, (uint64_t)j->qd.cap * 4);
@@ -2216,6 +2226,13 @@ extern "C" gst_status gst_query_noalloc(gst_graph* g, const uint32_t* groups, in
   const size_t o_ws = o;
   Layout L = layout_for(g, k, D, (size_t)n_members, max_edges);
   if (o_ws + L.total > GST_NOALLOC_SCRATCH_BYTES) return GST_SCRATCH_TOO_SMALL;
+  {
+    // there is no rerun with longer lists here, so the four lists share what is
+    // left of the scratch (less what aligning them may take)
+    const uint64_t spare = (GST_NOALLOC_SCRATCH_BYTES - o_ws - L.total) / 16;
+    const uint64_t want = std::min(L.cap + spare, std::min(list_bound(g, WT), list_cap_limit()));
+    if (want > (uint64_t)L.cap + 64) L = layout_for(g, k, D, (size_t)n_members, max_edges, want - 64);
+  }
 
   QDev* d_qd = reinterpret_cast<QDev*>(base + o_qd);
   QCtl* d_ctl = reinterpret_cast<QCtl*>(base + o_ctl);

@@ -144,7 +144,10 @@ gst_status gst_query_ratio(gst_graph* g, const uint32_t* groups, int k, int D, d
  * The call allocates no device or pinned host memory and issues its work on
  * the legacy default stream; it returns when the GPU work is done.
  *   - A query whose workspace does not fit returns GST_SCRATCH_TOO_SMALL
- *     (roughly: V * 2^k * (D+1) states need 8 + 16 + 2^-2 bytes each).
+ *     (roughly: V * 2^k * (D+1) states need 8 + 16 + 2^-2 bytes each).  Its
+ *     frontier lists take what is left of the array; a query that outgrows
+ *     them, which the other entry points rerun with longer ones, returns
+ *     GST_QUEUE_OVERFLOW.
  *   - The first call on a device looks up the array's device address
  *     (cudaGetSymbolAddress) with that device current; make that first call
  *     before any stream capture.
