@@ -1442,14 +1442,23 @@ struct DeviceTmp {
 };
 
 // Offsets, weight-sorted adjacency and weight-bucket index of a graph on its
-// device.  The arcs go over in pieces of ARC_PIECE, so the caller's separate
-// arrays never take more device memory than that beside the adjacency.
-constexpr size_t ARC_PIECE = 32u << 20;
-// Arcs of long lists merged together: bounds the merge's buffer (a longer list
-// is merged alone).
-constexpr size_t MERGE_GROUP = 32u << 20;
+// device.  What the work needs beside them lies in memory that is not filled yet:
+// the index's (V * 32 bytes), filled last, and, for the caller's arrays on their
+// way into the adjacency, the part of the adjacency that comes after.  So a graph
+// that fits is created also where the rest of the device is taken (a server holds
+// its whole budget), and there is nothing to free, which would wait for the work
+// of every engine.
+//
+// Merging is the exception, and only a wish: lists are merged in groups that fit
+// the index's memory with their copy, and each group costs some 30 us of copies
+// and launches.  A graph that would need more than MERGE_GROUPS of them (a dense
+// one) or has a list too long for it (parallel arcs) asks for up to MERGE_ARCS; a
+// list that fits nowhere is sorted on the host.
+constexpr size_t MERGE_GROUPS = 16;
+constexpr size_t MERGE_ARCS = 32u << 20;
 
 gst_status build_adjacency(gst_graph* g, const uint32_t* beg, const uint32_t* csr, const int32_t* w, ArcCheck& check) {
+  typedef unsigned long long u64;
   const uint32_t V = g->V;
   const uint64_t arcs = g->arcs;
   if (cudaMalloc(&g->d_beg, (size_t)(V + 1) * 4) != cudaSuccess ||
@@ -1460,66 +1469,86 @@ gst_status build_adjacency(gst_graph* g, const uint32_t* beg, const uint32_t* cs
   }
   CK(cudaMemcpy(g->d_beg, beg, (size_t)(V + 1) * 4, cudaMemcpyHostToDevice));
   const unsigned grid = (unsigned)g->num_sms * 8u;
-  if (arcs) {
-    const size_t piece = std::min<size_t>(arcs, ARC_PIECE);
-    DeviceTmp raw;
-    if (!raw.alloc(piece * 8)) return GST_OOM;
-    uint32_t* d_csr = static_cast<uint32_t*>(raw.p);
-    for (size_t a = 0; a < arcs; a += piece) {
-      const size_t n = std::min<size_t>(piece, arcs - a);
-      CK(cudaMemcpy(d_csr, csr + a, n * 4, cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(d_csr + piece, w + a, n * 4, cudaMemcpyHostToDevice));
-      k_pack_arcs<<<grid, 256>>>(d_csr, d_csr + piece, g->d_adj + a, n);
-      CK(cudaGetLastError());
-    }
-    CK(cudaStreamSynchronize(0));
+  u64* adj = reinterpret_cast<u64*>(g->d_adj);
+  u64* spare = reinterpret_cast<u64*>(g->d_wcut);
+  const size_t spare_words = (size_t)V * 4;
+  for (size_t a = 0; a < arcs;) {
+    // the two arrays of n arcs take as much as the n pairs: half of what is left
+    // goes by way of the other half's place, the last arcs by the index's
+    const size_t left = arcs - a, n = left <= spare_words ? left : left / 2;
+    uint32_t* raw = reinterpret_cast<uint32_t*>(left <= spare_words ? spare : adj + (arcs - n));
+    CK(cudaMemcpy(raw, csr + a, n * 4, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(raw + n, w + a, n * 4, cudaMemcpyHostToDevice));
+    k_pack_arcs<<<grid, 256>>>(raw, raw + n, g->d_adj + a, n);
+    CK(cudaGetLastError());
+    a += n;
   }
+  CK(cudaStreamSynchronize(0));
   if (!check.ok()) return GST_BAD_INPUT;
   g->wmax = check.heaviest();
-  unsigned long long* adj = reinterpret_cast<unsigned long long*>(g->d_adj);
   k_sort_lists<<<grid, 256>>>(g->d_beg, adj, V);
   CK(cudaGetLastError());
   // what no warp sorts: pieces for the blocks, and the long lists to merge
   std::vector<uint2> pieces, lists;
+  size_t longest = 0, total = 0;
   for (uint32_t v = 0; v < V; v++) {
     const uint32_t n = beg[v + 1] - beg[v];
     if (n <= 256u) continue;
-    for (uint32_t a = 0; a < n; a += SORT_BLOCK) pieces.push_back(make_uint2(beg[v] + a, std::min(SORT_BLOCK, n - a)));
-    if (n > SORT_BLOCK) lists.push_back(make_uint2(beg[v], n));
+    for (uint64_t a = 0; a < n; a += SORT_BLOCK)
+      pieces.push_back(make_uint2(beg[v] + (uint32_t)a, (uint32_t)std::min<uint64_t>(SORT_BLOCK, n - a)));
+    if (n <= SORT_BLOCK) continue;
+    lists.push_back(make_uint2(beg[v], n));
+    longest = std::max<size_t>(longest, n);
+    total += n;
   }
-  if (!pieces.empty()) {
-    DeviceTmp dp;
-    if (!dp.alloc(pieces.size() * sizeof(uint2))) return GST_OOM;
-    CK(cudaMemcpy(dp.p, pieces.data(), pieces.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-    k_sort_pieces<<<(unsigned)std::min<size_t>(pieces.size(), (size_t)g->num_sms * 4), 512>>>(
-        static_cast<const uint2*>(dp.p), (uint32_t)pieces.size(), adj);
+  for (size_t p = 0; p < pieces.size(); p += spare_words) {
+    const size_t n = std::min(spare_words, pieces.size() - p);
+    CK(cudaMemcpy(spare, pieces.data() + p, n * sizeof(uint2), cudaMemcpyHostToDevice));
+    k_sort_pieces<<<(unsigned)std::min<size_t>(n, (size_t)g->num_sms * 4), 512>>>(
+        reinterpret_cast<const uint2*>(spare), (uint32_t)n, adj);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(0));
+  }
+  // a group's words: its arcs' copy, its lists, and their offsets (32 bits, one more)
+  auto words = [](size_t arcs, size_t n) { return arcs + n + n / 2 + 1; };
+  DeviceTmp tmp;
+  u64* buf = spare;
+  size_t room = spare_words;
+  if (words(longest, 1) > room || total > MERGE_GROUPS * room) {
+    const size_t want = std::max(words(longest, 1), std::min(words(total, lists.size()), MERGE_ARCS));
+    if (tmp.alloc(want * 8)) {
+      buf = static_cast<u64*>(tmp.p);
+      room = want;
+    }
   }
   for (size_t l0 = 0; l0 < lists.size();) {
     std::vector<uint32_t> cum{0};
-    uint32_t longest = 0;
+    uint32_t top = 0;
     size_t l1 = l0;
-    for (; l1 < lists.size() && (l1 == l0 || cum.back() + (size_t)lists[l1].y <= MERGE_GROUP); l1++) {
+    for (; l1 < lists.size() && words((size_t)cum.back() + lists[l1].y, l1 + 1 - l0) <= room; l1++) {
       cum.push_back(cum.back() + lists[l1].y);
-      longest = std::max(longest, lists[l1].y);
+      top = std::max(top, lists[l1].y);
     }
     const size_t n = l1 - l0;
-    DeviceTmp tmp, dl;
-    if (!tmp.alloc((size_t)cum.back() * 8) || !dl.alloc(n * sizeof(uint2) + cum.size() * 4)) return GST_OOM;
-    uint2* d_list = static_cast<uint2*>(dl.p);
+    if (n == 0) {
+      const uint2 L = lists[l0++];
+      std::vector<u64> key(L.y);
+      for (uint32_t i = 0; i < L.y; i++) key[i] = (u64)(uint32_t)w[(size_t)L.x + i] << 32 | csr[(size_t)L.x + i];
+      std::sort(key.begin(), key.end());
+      CK(cudaMemcpy(adj + L.x, key.data(), key.size() * 8, cudaMemcpyHostToDevice));
+      continue;
+    }
+    uint2* d_list = reinterpret_cast<uint2*>(buf + cum.back());
     uint32_t* d_cum = reinterpret_cast<uint32_t*>(d_list + n);
     CK(cudaMemcpy(d_list, lists.data() + l0, n * sizeof(uint2), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_cum, cum.data(), cum.size() * 4, cudaMemcpyHostToDevice));
     int to_tmp = 1;
     uint64_t width = SORT_BLOCK;
-    for (; width < longest || !to_tmp; width *= 2) {  // an even number of passes ends in the adjacency
-      k_merge_runs<<<grid, 256>>>(d_list, d_cum, (uint32_t)n, adj, static_cast<unsigned long long*>(tmp.p),
-                                  (uint32_t)std::min<uint64_t>(width, 1u << 31), to_tmp);
+    for (; width < top || !to_tmp; width *= 2) {  // an even number of passes ends in the adjacency
+      k_merge_runs<<<grid, 256>>>(d_list, d_cum, (uint32_t)n, adj, buf, (uint32_t)std::min<uint64_t>(width, 1u << 31),
+                                  to_tmp);
       CK(cudaGetLastError());
       to_tmp ^= 1;
     }
-    CK(cudaStreamSynchronize(0));
     l0 = l1;
   }
   k_weight_index<<<grid, 256>>>(g->d_beg, g->d_adj, g->d_wcut, V);
@@ -2122,6 +2151,13 @@ gst_status gst_serve_stats(gst_server* S, gst_serve_info* out) {
   out->rejected_busy = S->n_busy;
   out->cancelled = S->n_cancelled;
   out->oom = S->n_oom;
+  return GST_OK;
+}
+
+gst_status gst_debug_adjacency(const gst_graph* g, uint32_t* pairs, uint32_t* index) {
+  if (!g || (!pairs && g->arcs) || !index) return GST_BAD_INPUT;
+  CK(cudaMemcpy(pairs, g->d_adj, g->arcs * 8, cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(index, g->d_wcut, (size_t)g->V * 32, cudaMemcpyDeviceToHost));
   return GST_OK;
 }
 

@@ -116,10 +116,12 @@ def lib():
         L.gst_serve_cancel.argtypes = [vp, u64]
         L.gst_serve_set_max_pending.argtypes = [vp, u64]
         L.gst_serve_stats.argtypes = [vp, ctypes.POINTER(_ServeInfo)]
+        L.gst_debug_adjacency.argtypes = [vp, vp, vp]
         L.gst_debug_fail_allocs.argtypes = [vp, ctypes.c_int]
         L.gst_debug_hold_rounds.argtypes = [vp, ctypes.c_int, ctypes.c_uint32]
         for name in ("gst_serve_open", "gst_serve_submit", "gst_serve_poll", "gst_serve_close", "gst_serve_cancel",
-                     "gst_serve_set_max_pending", "gst_serve_stats", "gst_debug_fail_allocs", "gst_debug_hold_rounds"):
+                     "gst_serve_set_max_pending", "gst_serve_stats", "gst_debug_adjacency", "gst_debug_fail_allocs",
+                     "gst_debug_hold_rounds"):
             getattr(L, name).restype = ctypes.c_int
         for name in ("gst_graph_create", "gst_groups_set", "gst_query", "gst_query_batch", "gst_query_batch_ratio",
                      "gst_query_ratio", "gst_serve_submit_ratio"):
@@ -194,6 +196,16 @@ class Engine:
         edges = buf[:3 * n].reshape(-1, 3).copy() if st in (GST_OK, GST_TRUNCATED) else np.zeros((0, 3), np.uint32)
         stats = {name: int(r.stats[i]) for i, name in enumerate(STAT_NAMES)}
         return QueryResult(st, r.cost, r.root, edges, stats, r.device_ms, r.latency_ms)
+
+    def adjacency(self):
+        """Test read-back (gst_debug_adjacency): the device's (arcs, 2) array of
+        {neighbour, weight} and its (V, 8) weight index."""
+        pairs = np.zeros((len(self._csr), 2), dtype=np.uint32)
+        index = np.zeros((self.V, 8), dtype=np.uint32)
+        st = lib().gst_debug_adjacency(self._h, _ptr(pairs), _ptr(index))
+        if st != GST_OK:
+            raise GstError(st, "gst_debug_adjacency")
+        return pairs, index
 
     def fail_allocs(self, n: int):
         """Fault injection: the next n workspace allocations fail (gst_debug_fail_allocs)."""

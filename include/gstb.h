@@ -270,6 +270,11 @@ gst_status gst_serve_stats(gst_server* s, gst_serve_info* out);
  * results not polled by then are discarded. */
 gst_status gst_serve_close(gst_server* s);
 
+/* Read-back for tests (no reference counterpart) of what gst_graph_create built
+ * on the device: pairs[2*arcs], {neighbour, weight} of every arc, each list
+ * sorted by (weight, neighbour); index[8*V], for each vertex the number of its
+ * first arc heavier than 2^b (b = 0..6), then of its first arc. */
+gst_status gst_debug_adjacency(const gst_graph* g, uint32_t* pairs, uint32_t* index);
 /* Fault injection for tests (no reference counterpart): the next n workspace
  * allocations of this graph's engines fail as if the device were full.  A
  * query that cannot be admitted while nothing else runs returns GST_OOM;
