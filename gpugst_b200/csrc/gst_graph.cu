@@ -7,9 +7,10 @@
 //                              by run: every element's place is its own index
 //                              plus its rank in the sibling run.
 // Measured on 170k vertices / 13.6M arcs: packing 0.04 ms, lists 0.28, pieces
-// 0.35, two merge passes 0.02 and the weight index 0.02; creating the graph went
-// from 102 to 16 ms, which is the copy of the caller's pageable arrays.  Bound by
-// the bitonic steps' shared-memory passes, which is no matter beside that copy.
+// 0.35, two merge passes 0.02 and the weight index 0.02; creating the graph, with a
+// sort on 16 host threads 105 ms, takes 16 (medians of 60), which is the copy of
+// the caller's pageable arrays.  Bound by the bitonic steps' shared-memory passes,
+// which is no matter beside that copy.
 #include "gst_device.cuh"
 
 namespace gstb {

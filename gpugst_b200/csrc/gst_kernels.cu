@@ -22,7 +22,7 @@
 //   split      near-far bucketing: far items whose cost entered the new
 //              window move to the near list
 //   tour       group-to-group distances and tour tables (host DP at
-//              DPQ.cu:409-483, re-done on device by one warp)
+//              DPQ.cu:409-483, re-done on device by a warp per starting group)
 //   seeds      members at distance 0 (DPQ.cu:359-368); cost-0 states of every
 //              subset of a member's group mask (DPQ.cu:341-358)
 //   extract    follow parents from the best full state into a tree (the
@@ -855,9 +855,9 @@ __device__ __forceinline__ void relax_flat(const QDev& q, const RelaxHdr* __rest
     // when that row showed the list's byte empty.  Within a round the
     // next-parity and far bytes only gain bits, so the first OR to reach a
     // byte comes from a lane that read it empty: every newly pending vertex
-    // is appended at least once.  Two lanes that both read it empty append
-    // it twice; the consumer's atomicAnd hands the groups to one of them
-    // and the other finds none.  No lane waits for an atomic's result.
+    // is appended at least once.  Every lane that read it empty appends it;
+    // the consumer's atomicAnd hands the groups to one of the entries and the
+    // others find none.  No lane waits for an atomic's result.
     uint32_t itv[SSSP_U];
     bool tN[SSSP_U], tF[SSSP_U];
 #pragma unroll
@@ -1106,7 +1106,9 @@ __device__ void grow_chunk(const QDev* qd, const uint4 item, const GraphDev& g, 
 // one at a time 4.1 -> 2.2 ms, 48 mixed queries on 3M vertices 202 -> 117 ms.
 //
 // Four items of the lists 0 .. D - b per warp, 8 lanes each; a vertex with at
-// least hub_min_deg arcs hands all but the first 32 to k_heavy in chunks.
+// least hub_min_deg arcs hands all but the first 32 to k_heavy in chunks.  With 4
+// and 16 lanes (queries one at a time, then 48 in a batch, on 2^20 vertices): 1579
+// and 1454 us against 1491, 2.98 and 2.88 ms against 2.94.
 // ---------------------------------------------------------------------------
 constexpr uint32_t CH_PULL = 1u << 29;  // big-list entry is a chunk of a gathered row
 constexpr uint32_t PULL_LANES = 8;
@@ -1836,8 +1838,9 @@ __device__ void init_rows(const QDev& q, const uint32_t* members, size_t tid, si
   // Unbounded queries have one buffer.  Of a hop-bounded query's two, the first is
   // read and written at the members only when there is one relaxed round
   // (D = 1..3), and the second not at all when there is none (D = 0).  Measured
-  // against both buffers always: one query (D = 2..4) on 2^20 vertices 1457 ->
-  // 1417 us, 48 in a batch 3.01 -> 2.86 ms; on 10k vertices the same.
+  // against both buffers always: six queries (D = 2..4) one at a time on 2^20
+  // vertices 1457 -> 1417 us, 48 in a batch 3.01 -> 2.86 ms; on 10k vertices the
+  // same.
   const bool first = q.push_rounds != 1u || members == nullptr;
   const bool second = next != dist && q.push_rounds != 0u;
   for (size_t i = tid; i < 2 * (size_t)q.nv; i += stride) {
@@ -2026,7 +2029,9 @@ __device__ __forceinline__ void hop_rounds_done(QRun& q, QDev& qg, QCtl& c, cons
 // all its arcs once more.  The reach took 90 queries on 170k vertices from 15.5 to
 // 14.8 ms and 48 mixed ones on 3M from 104 to 96; relaxing below the window's own
 // end only, with a look at every vertex for each new window, halved the arcs but
-// cost the serving mixes 2-6%.
+// cost the serving mixes 2-6%.  LIGHT_ITEMS is some four items a warp of the whole
+// GPU; a quarter of it costs two queries of k = 6, 7 on 54k vertices 1% (2942 us
+// against 2915), four times as many changes nothing.
 constexpr uint32_t LIGHT_ITEMS = 16384;
 __device__ __forceinline__ uint32_t window_end(const QRun& q, uint32_t lo, uint32_t best, uint32_t limit) {
   uint32_t w = q.delta;
@@ -2164,7 +2169,13 @@ __device__ __forceinline__ void decide(QRun& q, QDev& qg, QCtl& c, const CtlIn& 
   }
 }
 
-// Bounds of a small round, per warp of the cluster (k_small).
+// Bounds of a small round, per warp of the cluster (k_small).  Half and twice each,
+// against these: one k = 4 query on 10k vertices through the allocation-free call
+// (no arc chunks, launches not in a graph) 551 and 533 us for SMALL_ARCS, 554 and
+// 531 for SMALL_DP, 556 and 533 for SMALL_TASKS (532); four hop-bounded ones there
+// 1158 and 1181, 1176 and 1169, 1190 and 1164 (1166); two of k = 6, 7 on 54k
+// vertices 2953 and 2873, 2927 and 2899, 2902 and 2915 (2915); SMALL_CHUNKS, and
+// all four on 170k and 2^20 vertices, within 1.1%.
 constexpr uint32_t SMALL_ARCS = 256, SMALL_DP = 2, SMALL_TASKS = 2, SMALL_CHUNKS = 4;
 
 // Shared memory of one control step.
